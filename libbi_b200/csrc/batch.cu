@@ -7,10 +7,11 @@
 // filters of one model (each with its own particle count, constants, seed and
 // resampler) in shared structure-of-arrays buffers, and one filter step of
 // the whole batch is two launches:
-//   k_batch_resample      one 1024-thread CTA per filter that resamples
+//   k_batch_resample      one cluster of eight CTAs per filter that resamples
 //                         (gated on the filter's own ESS flag): the permuted
 //                         systematic, multinomial or Metropolis ancestors of
 //                         the single-filter path, computed on chip
+//                         (batch_resample.cu)
 //   k_batch_*_transition  one thread per particle over all filters' blocks;
 //                         the last block of each filter finalises that
 //                         filter's ESS, lW, logLikelihood and resample flag
@@ -32,8 +33,6 @@
 #include <vector>
 
 namespace bpf {
-
-constexpr int kBatchThreads = 1024;
 
 // ---------------------------------------------------------------------------
 // initial draws (Simulator::init -> Model::initialSamples) and statistics
@@ -164,243 +163,6 @@ k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld,
 }
 
 // ---------------------------------------------------------------------------
-// resampling, one CTA per filter
-// ---------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ int block_exclusive_max_int_nt(int v, int* total) {
-  __shared__ int wt[NT / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int inc = v;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    int o = __shfl_up_sync(0xffffffffu, inc, d);
-    if (lane >= d) inc = max(inc, o);
-  }
-  const int excl_in_warp = __shfl_up_sync(0xffffffffu, inc, 1);
-  if (lane == 31) wt[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    int t = lane < NT / 32 ? wt[lane] : 0;
-#pragma unroll
-    for (int d = 1; d < NT / 32; d <<= 1) {
-      int o = __shfl_up_sync(0xffffffffu, t, d);
-      if (lane >= d) t = max(t, o);
-    }
-    if (lane < NT / 32) wt[lane] = t;
-  }
-  __syncthreads();
-  int r = warp > 0 ? wt[warp - 1] : 0;
-  if (lane > 0) r = max(r, excl_in_warp);
-  *total = wt[NT / 32 - 1];
-  __syncthreads();
-  return r;
-}
-
-__device__ __forceinline__ unsigned long long batch_q(const double* lwf, int i, double mx) {
-  return weight_to_fixed(nanexp(__dsub_rn(__ldg(lwf + i), mx)));
-}
-
-__device__ __forceinline__ u128 u128_of(unsigned long long q) {
-  u128 r; r.lo = q; r.hi = 0; return r;
-}
-
-// Number of entries of the nondecreasing lu[0..n) below x: a binary search
-// over every 32nd entry (in shared memory), then over one run of 32 in L2.
-__device__ __forceinline__ int count_below(const double* lu, const double* s_coarse, int nc, int n, double x) {
-  int lo = 0, hi = nc;  // first coarse c with lu[32c] >= x
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (s_coarse[mid] < x) lo = mid + 1; else hi = mid;
-  }
-  // answer in (32(lo-1), 32 lo], clipped to [0, n]
-  int a = lo > 0 ? 32 * (lo - 1) + 1 : 0;
-  int b = min(n, 32 * lo);
-  while (a < b) {
-    const int mid = (a + b) >> 1;
-    if (__ldcg(lu + mid) < x) a = mid + 1; else b = mid;
-  }
-  return a;
-}
-
-// Shared memory: marks (one int per particle), childless flags (one byte per
-// particle), coarse multinomial index (kBatchThreads doubles).
-inline size_t batch_resample_smem(int max_n) {
-  return (size_t)max_n * sizeof(int) + (size_t)max_n + (size_t)kBatchThreads * sizeof(double) + 16;
-}
-
-// Batches whose largest filter has at most kBatchOsSmemMax particles keep
-// the cumulative offspring in shared memory too (the SMEM_OS kernels): the
-// CTA's passes over them then cost shared-memory latency instead of L2
-// round trips
-constexpr int kBatchOsSmemMax = 12288;
-inline size_t batch_resample_smem_os(int max_n) { return batch_resample_smem(max_n) + (size_t)max_n * sizeof(int); }
-
-template <bool SMEM_OS>
-__device__ __forceinline__ int ld_os(const int* p) {
-  if constexpr (SMEM_OS) return *p;
-  else return __ldcg(p);
-}
-
-// Permuted ancestors of filter blockIdx.x, the rule of
-// ResamplerHost::cumulativeOffspringToAncestorsPermute
-// (share/src/bi/host/resampler/ResamplerHost.hpp:134-168) in closed form:
-// survivors in place, extra copies by ancestor into the childless slots in
-// ascending order.  Cumulative offspring of
-//   systematic   SystematicResampler::cumulativeOffspring (SystematicResampler.hpp:111-130)
-//   multinomial  MultinomialResamplerHost::ancestors (MultinomialResamplerHost.hpp:29-65)
-//   Metropolis   MetropolisResamplerHost::ancestors (MetropolisResamplerHost.hpp:32-62)
-// computed exactly as the single-filter kernels compute them.
-template <int NT, bool SMEM_OS>
-__global__ void __launch_bounds__(NT, 1)
-k_batch_resample(const double* __restrict__ lw, int* __restrict__ as, const BatchFilter* __restrict__ filt,
-                 const int* __restrict__ order, StepStats* stats, double* lu_buf, int* os_buf, int step) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
-  pdl_trigger();  // a single filter's transition, a programmatic dependent, may be scheduled
-  const int f = order[blockIdx.x];
-  const BatchFilter fd = filt[f];
-  StepStats* st = stats + f;
-  if (st->resample == 0 || st->status != BPF_OK) return;  // uniform over the block
-  const int n = fd.n;
-  const double* lwf = lw + fd.off;
-  int* asf = as + fd.off;
-  double* s_coarse = reinterpret_cast<double*>(s_raw);
-  int* marks = reinterpret_cast<int*>(s_raw + kBatchThreads * sizeof(double));  // layout for the largest NT
-  // the cumulative offspring: after the marks in shared memory, or the
-  // filter's columns of the global buffer
-  int* osf = SMEM_OS ? marks + n : os_buf + fd.off;
-  unsigned char* flags = reinterpret_cast<unsigned char*>(SMEM_OS ? osf + n : marks + n);
-  const int IT = (n + NT - 1) / NT;
-  const int i0 = min(n, threadIdx.x * IT);
-  const int i1 = min(n, i0 + IT);
-  const double mx = st->mx;
-  const double nd = (double)n;
-
-  // ---- cumulative offspring Os of this thread's particles, into osf ----
-  if (fd.resampler == BPF_RESAMPLER_SYSTEMATIC || fd.resampler == BPF_RESAMPLER_MULTINOMIAL) {
-    const bool mult = fd.resampler == BPF_RESAMPLER_MULTINOMIAL;
-    u128 acc = u128_zero(), vacc = u128_zero();
-    for (int i = i0; i < i1; ++i) {
-      acc = u128_add(acc, u128_of(batch_q(lwf, i, mx)));
-      if (mult) vacc = u128_add(vacc, spacing_to_fixed(multinomial_spacing(nullptr, i, n, fd.seed, step)));
-    }
-    u128 Wtot;
-    const u128 texcl = block_exclusive_scan_u128_nt<NT>(acc, &Wtot);
-    const double W = u128_to_weight(Wtot);
-    // SystematicResampler::cumulativeOffspring throws
-    // ParticleFilterDegeneratedException unless W > 0
-    // (share/src/bi/resampler/SystematicResampler.hpp:118-129)
-    if (!(W > 0.0)) {
-      if (threadIdx.x == 0) st->status = BPF_E_DEGENERATE;
-      return;
-    }
-    if (!mult) {
-      bpf_u32x4 r = bpf_draw(fd.seed, 0u, (uint32_t)step, 0u, BPF_RNG_SYSTEMATIC);
-      const double a = bpf_u01d(r.v[0], r.v[1]);
-      const double yW = __ddiv_rn(1.0, W);
-      u128 Q = texcl;
-      for (int i = i0; i < i1; ++i) {
-        Q = u128_add(Q, u128_of(batch_q(lwf, i, mx)));
-        osf[i] = systematic_Os(u128_to_weight(Q), W, yW, nd, a, n);
-      }
-    } else {
-      u128 Vtot;
-      const u128 vexcl = block_exclusive_scan_u128_nt<NT>(vacc, &Vtot);
-      const double lW = log(W);
-      double* luf = lu_buf + fd.off;
-      // lu_s = lW + lMax_s, lMax_s = -(sum of the spacings of slots >= s)
-      u128 V = vexcl;
-      for (int s = i0; s < i1; ++s) {
-        const double lu = __dadd_rn(lW, -fixed_to_spacing(u128_sub(Vtot, V)));
-        luf[s] = lu;
-        if ((s & 31) == 0) s_coarse[s >> 5] = lu;
-        V = u128_add(V, spacing_to_fixed(multinomial_spacing(nullptr, s, n, fd.seed, step)));
-      }
-      __syncthreads();
-      const int nc = (n + 31) >> 5;
-      // slot s takes the number of m with log(Ws_m) <= lu_s (clamped to n-1),
-      // so Os_m = #{s : lu_s < log(Ws_m)} for m < n-1 and Os_{n-1} = n
-      u128 Q = texcl;
-      for (int m = i0; m < i1; ++m) {
-        Q = u128_add(Q, u128_of(batch_q(lwf, m, mx)));
-        osf[m] = m == n - 1 ? n : count_below(luf, s_coarse, nc, n, log(u128_to_weight(Q)));
-      }
-    }
-  } else {
-    // Metropolis: B steps per particle, then offspring counts and their
-    // cumulative sums in place
-    for (int i = i0; i < i1; ++i) osf[i] = 0;
-    __syncthreads();
-    for (int p = i0; p < i1; ++p) {
-      const int a = metropolis_ancestor(lwf, n, fd.B, nullptr, fd.seed, step, p);
-      atomicAdd(osf + a, 1);
-    }
-    __syncthreads();
-    int loc = 0;
-    for (int i = i0; i < i1; ++i) loc += ld_os<SMEM_OS>(osf + i);
-    int tot;
-    int run = block_exclusive_scan_int_nt<NT>(loc, &tot);
-    for (int i = i0; i < i1; ++i) { run += ld_os<SMEM_OS>(osf + i); osf[i] = run; }
-  }
-  __syncthreads();
-
-  // ---- permutation: childless counts, survivors, extra-copy marks ----
-  const int before0 = i0 == 0 ? 0 : ld_os<SMEM_OS>(osf + i0 - 1);
-  int zl = 0;
-  {
-    int prev = before0;
-    for (int i = i0; i < i1; ++i) {
-      const int o = ld_os<SMEM_OS>(osf + i);
-      zl += (o == prev);
-      prev = o;
-    }
-  }
-  int ztot;
-  const int zexcl = block_exclusive_scan_int_nt<NT>(zl, &ztot);
-  for (int r = threadIdx.x; r < ztot; r += NT) marks[r] = 0;
-  __syncthreads();
-  {
-    int prev = before0, Z = zexcl;
-    for (int i = i0; i < i1; ++i) {
-      const int o = ld_os<SMEM_OS>(osf + i);
-      const bool zero = o == prev;
-      flags[i] = zero;
-      if (!zero) {
-        asf[i] = i;
-        // E_i = Os_{i-1} - i + Z_i extra copies precede particle i's
-        const int e = prev - i + Z;
-        if (o - prev >= 2 && e >= 0 && e < ztot) marks[e] = i + 1;
-      }
-      Z += zero;
-      prev = o;
-    }
-  }
-  __syncthreads();
-  // inclusive max-scan of marks[0..ztot): rank r -> 1 + the ancestor whose
-  // extra copies cover r
-  {
-    const int CH = (ztot + NT - 1) / NT;
-    const int r0 = min(ztot, threadIdx.x * CH), r1 = min(ztot, r0 + CH);
-    int m = 0;
-    for (int r = r0; r < r1; ++r) m = max(m, marks[r]);
-    int mtot;
-    const int mexcl = block_exclusive_max_int_nt<NT>(m, &mtot);
-    int run = mexcl;
-    for (int r = r0; r < r1; ++r) { run = max(run, marks[r]); marks[r] = run; }
-  }
-  __syncthreads();
-  {
-    int Z = zexcl;
-    for (int i = i0; i < i1; ++i)
-      if (flags[i]) {
-        // a consistent Os gives 1 <= marks[Z] <= n; anything else stays in range
-        const int a = Z < ztot ? marks[Z] - 1 : i;
-        asf[i] = a >= 0 && a < n ? a : i;
-        ++Z;
-      }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 int launch_batch_init(const ModelArgs& m, void* x, int ld, double* lw, const BatchFilter* filt, const void* prms,
@@ -454,162 +216,6 @@ int launch_batch_transition(const ModelArgs& m, const void* x_in, void* x_out, i
   return BPF_OK;
 }
 
-// threads per filter CTA of the batched resampler: 256, 512 or 1024 (the
-// in-CTA arithmetic is exact, so the count changes the speed only)
-int launch_batch_resample(const double* lw, int* as, const BatchFilter* filt, const int* order, int nf,
-                          int max_n, StepStats* stats, double* lu_buf, int* os_buf, int step, cudaStream_t st,
-                          int threads) {
-  if (max_n <= kBatchOsSmemMax) {
-    const size_t smem = batch_resample_smem_os(max_n);
-    switch (threads) {
-      case 256:
-        k_batch_resample<256, true><<<nf, 256, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      case 512:
-        k_batch_resample<512, true><<<nf, 512, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      case 1024:
-        k_batch_resample<1024, true><<<nf, 1024, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      default: return BPF_E_INVALID;
-    }
-  } else {
-    const size_t smem = batch_resample_smem(max_n);
-    switch (threads) {
-      case 256:
-        k_batch_resample<256, false><<<nf, 256, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      case 512:
-        k_batch_resample<512, false><<<nf, 512, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      case 1024:
-        k_batch_resample<1024, false><<<nf, 1024, smem, st>>>(lw, as, filt, order, stats, lu_buf, os_buf, step);
-        break;
-      default: return BPF_E_INVALID;
-    }
-  }
-  BPF_TRY(cudaGetLastError());
-  return BPF_OK;
-}
-
-// The limit is a property of the kernel, shared by every batch: it is raised
-// to what the largest allowed filter needs (a smaller batch created later
-// must not lower it under a larger one), once per device.
-int configure_batch_resample(int max_n) {
-  if (max_n > BPF_BATCH_MAX_PARTICLES) return BPF_E_INVALID;
-  static unsigned c256 = 0, c512 = 0, c1024 = 0, d256 = 0, d512 = 0, d1024 = 0;
-  const int smem = (int)batch_resample_smem(BPF_BATCH_MAX_PARTICLES);
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<256, false>, smem, c256));
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<512, false>, smem, c512));
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<1024, false>, smem, c1024));
-  const int smem_os = (int)batch_resample_smem_os(kBatchOsSmemMax);
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<256, true>, smem_os, d256));
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<512, true>, smem_os, d512));
-  BPF_TRY(set_dyn_smem_once(k_batch_resample<1024, true>, smem_os, d1024));
-  return BPF_OK;
-}
-
-// synthetic log-weights 2 N(0, 1) over the whole buffer, for the autotuner
-__global__ void k_batch_synthetic_lw(double* lw, int ld) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ld) return;
-  const bpf_u32x4 r = bpf_draw(0x7a11ull, (uint32_t)i, 0u, 0u, BPF_RNG_DATA);
-  double z0, z1;
-  bpf_normal_pair_d(r.v[0], r.v[1], &z0, &z1);
-  lw[i] = 2.0 * z0;
-}
-
-// statistics that open every filter's resampling gate, with each filter's
-// maximum log-weight
-__global__ void k_batch_tune_stats(const double* lw, const BatchFilter* filt, StepStats* st, int nf) {
-  const int f = blockIdx.x;
-  if (f >= nf) return;
-  const BatchFilter fd = filt[f];
-  double m = -INFINITY;
-  for (int i = threadIdx.x; i < fd.n; i += blockDim.x) m = fmax(m, lw[fd.off + i]);
-  m = warp_max(m);
-  __shared__ double s_m[32];
-  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, s_m[w]);
-    m = fmax(m, s_m[0]);
-    StepStats z{};
-    z.mx = m;
-    z.resample = 1;
-    z.status = BPF_OK;
-    z.n = fd.n;
-    st[f] = z;
-  }
-}
-
-// Time the three thread counts on synthetic log-weights laid out as the
-// batch's filters (scratch buffers: the batch's own state is untouched) and
-// return the fastest; the medians go to us[3] (256, 512, 1024).
-int tune_batch_resample(const BatchFilter* filt, const int* order, int nf, int max_n, int ld, cudaStream_t st,
-                        int* best, double* us) {
-  *best = kBatchThreads;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  BPF_TRY(cudaStreamIsCapturing(st, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return BPF_OK;  // no timing inside a capture: keep the default
-  double* lw = nullptr;
-  double* lu = nullptr;
-  int *as = nullptr, *os = nullptr;
-  StepStats* stats = nullptr;
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  int rc = BPF_OK;
-  auto A = [&](void** p, size_t b) {
-    if (!rc && cudaMalloc(p, b) != cudaSuccess) rc = BPF_E_NOMEM;
-  };
-  A((void**)&lw, (size_t)ld * sizeof(double));
-  A((void**)&lu, (size_t)ld * sizeof(double));
-  A((void**)&as, (size_t)ld * sizeof(int));
-  A((void**)&os, (size_t)ld * sizeof(int));
-  A((void**)&stats, (size_t)nf * sizeof(StepStats));
-  if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = BPF_E_CUDA;
-  if (!rc) {
-    k_batch_synthetic_lw<<<(ld + 255) / 256, 256, 0, st>>>(lw, ld);
-    k_batch_tune_stats<<<nf, 256, 0, st>>>(lw, filt, stats, nf);
-    if (cudaGetLastError() != cudaSuccess) rc = BPF_E_CUDA;
-  }
-  // the sizes take turns, round after round, so that a drift of clocks or
-  // caches during the tuning reaches every size alike; each size's median
-  // decides
-  const int counts[3] = {256, 512, 1024};
-  constexpr int kReps = 9;
-  float t[3][kReps];
-  for (int r = -2; !rc && r < kReps; ++r) {  // two untimed rounds first
-    for (int c = 0; !rc && c < 3; ++c) {
-      if (r >= 0 && cudaEventRecord(e0, st) != cudaSuccess) { rc = BPF_E_CUDA; break; }
-      rc = launch_batch_resample(lw, as, filt, order, nf, max_n, stats, lu, os, 1, st, counts[c]);
-      if (!rc && r >= 0 &&
-          (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-           cudaEventElapsedTime(&t[c][r], e0, e1) != cudaSuccess))
-        rc = BPF_E_CUDA;
-    }
-  }
-  double best_us = 0.0;
-  for (int c = 0; !rc && c < 3; ++c) {
-    std::sort(t[c], t[c] + kReps);
-    const double med = 1e3 * t[c][kReps / 2];
-    if (us) us[c] = med;
-    if (c == 0 || med < best_us) {
-      best_us = med;
-      *best = counts[c];
-    }
-  }
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
-  void* ps[] = {lw, lu, as, os, stats};
-  for (void* q : ps)
-    if (q) cudaFree(q);
-  if (rc) {
-    cudaGetLastError();
-    *best = kBatchThreads;
-  }
-  return rc;
-}
-
 }  // namespace bpf
 
 // ---------------------------------------------------------------------------
@@ -617,10 +223,9 @@ int tune_batch_resample(const BatchFilter* filt, const int* order, int nf, int m
 // ---------------------------------------------------------------------------
 struct bpf_batch {
   bpf::ModelArgs model;
-  int nf = 0, ld = 0, blocks = 0, max_n = 0, esz = 0, nobs = 0, bs = 0;
+  int nf = 0, ld = 0, blocks = 0, esz = 0, nobs = 0, bs = 0;
   int tiles = 0;               // 128-particle tiles over all filters (guided step)
-  int rs_threads = 1024;       // threads per filter CTA of the resampler (autotuned at create)
-  double rs_us[3] = {0.0, 0.0, 0.0};  // its tuning medians for 256, 512, 1024 threads
+  double rs_us[3] = {0.0, 0.0, 0.0};  // the resampler's tuning medians for 256, 512, 1024 threads
   bpf_proposal* prop = nullptr;  // learned proposal (bpf_batch_set_proposal), owned by the caller
   int* tile2f = nullptr;       // tile -> filter, allocated with the proposal
   // the PZ guided step's network outputs (ld entries), allocated with a PZ proposal
@@ -640,7 +245,10 @@ struct bpf_batch {
   bpf::BatchFilter* filt_dev = nullptr;
   void* prm_dev = nullptr;
   int* blk2f = nullptr;
-  int* order = nullptr;
+  int* order = nullptr;        // the filters, the largest first
+  bpf::BatchFilter* sorted = nullptr;  // and their entries in that order
+  std::vector<int> order_host;
+  bpf::ResamplePlan rs;        // cluster size and threads of the resampler (autotuned at create)
   double* lu = nullptr;
   int* os = nullptr;
   void* y_dev = nullptr;
@@ -688,6 +296,17 @@ int batch_upload_params(bpf_batch* b) {
   return upload_params(b, v);
 }
 
+// the filters' entries, and the same in the resampler's order
+int upload_filters(bpf_batch* b) {
+  std::vector<bpf::BatchFilter> sorted((size_t)b->nf);
+  for (int k = 0; k < b->nf; ++k) sorted[k] = b->filt[b->order_host[k]];
+  const size_t bytes = sorted.size() * sizeof(bpf::BatchFilter);
+  BPF_TRY(cudaMemcpyAsync(b->filt_dev, b->filt.data(), bytes, cudaMemcpyHostToDevice, b->stream));
+  BPF_TRY(cudaMemcpyAsync(b->sorted, sorted.data(), bytes, cudaMemcpyHostToDevice, b->stream));
+  BPF_TRY(cudaStreamSynchronize(b->stream));  // sorted is a temporary
+  return BPF_OK;
+}
+
 int batch_check_theta(const bpf_model_desc* m, const double* th) {
   if (m->kind == BPF_MODEL_L96) {
     if (!(th[1] >= 0.0) || !(th[2] > 0.0)) return BPF_E_INVALID;
@@ -702,7 +321,7 @@ void batch_free(bpf_batch* b) {
   for (cudaEvent_t e : b->ev)
     if (e) cudaEventDestroy(e);
   void* ptrs[] = {b->x[0], b->x[1], b->lw, b->as, b->stats, b->partials, b->counters, b->filt_dev,
-                  b->prm_dev, b->blk2f, b->order, b->lu, b->os, b->y_dev, b->hist, b->tile2f,
+                  b->prm_dev, b->blk2f, b->order, b->sorted, b->lu, b->os, b->y_dev, b->hist, b->tile2f,
                   b->gO};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -728,8 +347,7 @@ int batch_enqueue_init(bpf_batch* b) {
 
 int batch_enqueue_step(bpf_batch* b, double t1, double t2, const void* y_dev, double* hist, int k) {
   const int step = b->step + 1;
-  int rc = bpf::launch_batch_resample(b->lw, b->as, b->filt_dev, b->order, b->nf, b->max_n, b->stats, b->lu,
-                                      b->os, step, b->stream, b->rs_threads);
+  int rc = bpf::launch_batch_resample(b->lw, b->as, b->rs, b->stats, b->lu, b->os, step, b->stream);
   if (rc) return rc;
   if (b->prop && y_dev && b->model.kind == BPF_MODEL_PZ) {
     // guided step of the PZ model: the proposal over the log-noise
@@ -871,14 +489,15 @@ int bpf_batch_create(const bpf_model_desc* model, int nfilters, const bpf_batch_
     for (int i = 0; i < BPF_MAX_THETA; ++i) b->theta[(size_t)f * BPF_MAX_THETA + i] = bf.theta[i];
     for (int k = 0; k < d.nblocks; ++k) blk2f.push_back(f);
     off += d.nblocks * b->bs;
-    b->max_n = std::max(b->max_n, d.n);
   }
   b->ld = off;
   b->blocks = (int)blk2f.size();
   // largest filters resample first
-  std::vector<int> order((size_t)nfilters);
+  std::vector<int>& order = b->order_host;
+  order.resize((size_t)nfilters);
   for (int f = 0; f < nfilters; ++f) order[f] = f;
   std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return b->filt[i].n > b->filt[j].n; });
+  bpf::plan_batch_resample(b->filt.data(), nfilters, &b->rs);
 
   int rc = BPF_OK;
   if (stream) {
@@ -903,21 +522,21 @@ int bpf_batch_create(const bpf_model_desc* model, int nfilters, const bpf_batch_
   if (!rc) rc = dalloc(&b->prm_dev, (size_t)nfilters * prm_b);
   if (!rc) rc = dalloc(&b->blk2f, (size_t)b->blocks * sizeof(int));
   if (!rc) rc = dalloc(&b->order, (size_t)nfilters * sizeof(int));
+  if (!rc) rc = dalloc(&b->sorted, (size_t)nfilters * sizeof(bpf::BatchFilter));
   if (!rc) rc = dalloc(&b->lu, L * sizeof(double));
   if (!rc) rc = dalloc(&b->os, L * sizeof(int));
   if (!rc && (cudaMemsetAsync(b->counters, 0, (size_t)nfilters * sizeof(unsigned), b->stream) != cudaSuccess ||
               cudaMemsetAsync(b->as, 0, L * sizeof(int), b->stream) != cudaSuccess ||
-              cudaMemcpyAsync(b->filt_dev, b->filt.data(), b->filt.size() * sizeof(bpf::BatchFilter),
-                              cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
               cudaMemcpyAsync(b->blk2f, blk2f.data(), blk2f.size() * sizeof(int), cudaMemcpyHostToDevice,
                               b->stream) != cudaSuccess ||
               cudaMemcpyAsync(b->order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice,
                               b->stream) != cudaSuccess ||
               cudaStreamSynchronize(b->stream) != cudaSuccess))
     rc = BPF_E_CUDA;
-  if (!rc) rc = bpf::configure_batch_resample(b->max_n);
-  if (!rc) rc = bpf::tune_batch_resample(b->filt_dev, b->order, b->nf, b->max_n, b->ld, b->stream, &b->rs_threads,
-                                         b->rs_us);
+  if (!rc) rc = upload_filters(b);
+  b->rs.order = b->order;
+  b->rs.sorted = b->sorted;
+  if (!rc) rc = bpf::tune_batch_resample(b->filt_dev, &b->rs, b->ld, b->stream, b->rs_us);
   if (!rc) rc = batch_upload_params(b);
   if (!rc) rc = batch_enqueue_init(b);
   if (rc) {
@@ -1007,13 +626,13 @@ int bpf_batch_resample_threads(bpf_batch* b, int threads, int* current, double* 
   if (!b) return BPF_E_INVALID;
   if (threads != 0) {
     if (threads != 256 && threads != 512 && threads != 1024) return BPF_E_INVALID;
-    if (threads != b->rs_threads && b->graph) {
+    if (threads != b->rs.threads && b->graph) {
       cudaGraphExecDestroy(b->graph);  // the captured steps launch the other count
       b->graph = nullptr;
     }
-    b->rs_threads = threads;
+    b->rs.threads = threads;
   }
-  if (current) *current = b->rs_threads;
+  if (current) *current = b->rs.threads;
   if (tuned_us)
     for (int c = 0; c < 3; ++c) tuned_us[c] = b->rs_us[c];
   return BPF_OK;
@@ -1022,10 +641,7 @@ int bpf_batch_resample_threads(bpf_batch* b, int threads, int* current, double* 
 int bpf_batch_set_seeds(bpf_batch* b, const uint64_t* seeds) {
   if (!b || !seeds) return BPF_E_INVALID;
   for (int f = 0; f < b->nf; ++f) b->filt[f].seed = seeds[f];
-  BPF_TRY(cudaMemcpyAsync(b->filt_dev, b->filt.data(), b->filt.size() * sizeof(bpf::BatchFilter),
-                          cudaMemcpyHostToDevice, b->stream));
-  BPF_TRY(cudaStreamSynchronize(b->stream));
-  return BPF_OK;
+  return upload_filters(b);
 }
 
 int bpf_batch_step_device(bpf_batch* b, double t1, double t2, const void* y_device) {

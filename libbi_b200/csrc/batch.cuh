@@ -29,12 +29,21 @@ __device__ __forceinline__ void batch_record(const StepStats* st, double* hist, 
   }
 }
 
-// the batched resampler (batch.cu): one CTA of `threads` threads per filter
-int launch_batch_resample(const double* lw, int* as, const BatchFilter* filt, const int* order, int nf,
-                          int max_n, StepStats* stats, double* lu_buf, int* os_buf, int step, cudaStream_t st,
-                          int threads);
-int configure_batch_resample(int max_n);
-int tune_batch_resample(const BatchFilter* filt, const int* order, int nf, int max_n, int ld, cudaStream_t st,
-                        int* best, double* us);
+// the batched resampler (batch_resample.cu): how a batch's filters are
+// resampled
+struct ResamplePlan {
+  const int* order = nullptr;           // the filters, the largest first (device)
+  const BatchFilter* sorted = nullptr;  // their entries in that order (device)
+  int nf = 0;
+  int max_n = 0;      // particles of the largest filter
+  bool mult = false;  // any multinomial resampler
+  int group = 1;      // CTAs per filter (one thread-block cluster)
+  int threads = 1024; // per CTA
+};
+// fills all of the plan but order and sorted
+void plan_batch_resample(const BatchFilter* filt, int nf, ResamplePlan* p);
+int launch_batch_resample(const double* lw, int* as, const ResamplePlan& p, StepStats* stats, double* lu_buf,
+                          int* os_buf, int step, cudaStream_t st);
+int tune_batch_resample(const BatchFilter* filt, ResamplePlan* p, int ld, cudaStream_t st, double* us);
 
 }  // namespace bpf

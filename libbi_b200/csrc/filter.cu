@@ -17,6 +17,7 @@
 #include <mutex>
 #include <cstring>
 #include <new>
+#include <tuple>
 #include <cmath>
 #include <vector>
 
@@ -52,12 +53,12 @@ struct bpf_handle {
   bpf_proposal* prop = nullptr;
   // pinned host copy of the step statistics (read back after every step)
   bpf::StepStats* host_stats = nullptr;
-  // filters of at most kOneCtaMaxParticles resample in one CTA: the
+  // small filters resample in one thread-block cluster: the
   // batched resampler on a one-filter table (same ancestors, no grid
   // barriers); its CTA size is autotuned at create
   bpf::BatchFilter* one_filt = nullptr;
   int* one_order = nullptr;
-  int one_threads = 1024;
+  bpf::ResamplePlan one_plan;
   // path cache (bpf_path_cache): the pruned ancestry of the particles since
   // the record started (pc_len generations), at most pc_cap steps
   bpf::AncestryPool pc;
@@ -278,8 +279,7 @@ int enqueue_step(bpf_handle* h, double t1, double t2, const void* y_dev, uint64_
   ra.Os_out = nullptr;
   ra.gate = gate;
   ra.max_known = true;
-  int rc = h->one_filt ? bpf::launch_batch_resample(h->lw, h->as, h->one_filt, h->one_order, 1, h->n, h->rs.stats,
-                                                    h->rs.lu, h->rs.Os, k, h->stream, h->one_threads)
+  int rc = h->one_filt ? bpf::launch_batch_resample(h->lw, h->as, h->one_plan, h->rs.stats, h->rs.lu, h->rs.Os, k, h->stream)
                        : bpf::launch_resample(ra, h->rs, h->stream);
   if (rc) return rc;
   if (y_host && y_dev) BPF_TRY(cudaMemcpyAsync(const_cast<void*>(y_dev), y_host, y_bytes, cudaMemcpyHostToDevice,
@@ -377,32 +377,39 @@ __global__ void k_reset_lw(double* lw, int n, const bpf::StepStats* st) {
 
 }  // namespace
 
-// Largest filter resampled by one CTA.  On B200 (L96, d=40, a resampling
-// at every step) one CTA takes 9.6 / 12.3 / 16.4 us per systematic
-// resampling at N = 256 / 1024 / 4096 against 13.7 / 14.3 / 17.3 us for the
-// grid-wide kernels (Metropolis at 4096: 14.3 against 29.8 us), but 62 us
-// at 16384 against 17.8: past a few thousand particles the work needs more
-// than one SM.
-constexpr int kOneCtaMaxParticles = 4096;
+// The largest filter resampled by one cluster (the batched resampler on a
+// one-filter table) instead of the grid-wide kernels.  Per step of a plankton
+// filter (transition included, resampled at every step), one cluster against
+// the grid-wide kernels on B200: systematic 17.7 / 19.1 / 21.6 us against
+// 21.8 / 20.2 / 21.6 at N = 4096 / 8192 / 16384, multinomial 25 / 40 / 42
+// against 41 / 42 / 44 at 8192 / 16384 / 32768, Metropolis (16 steps) 27 / 36
+// us against 30 / 32 at 4096 / 8192: past these sizes eight SMs are too few.
+static int cluster_max_particles(int resampler) {
+  return resampler == BPF_RESAMPLER_METROPOLIS ? 4096 : resampler == BPF_RESAMPLER_MULTINOMIAL ? 32768 : 8192;
+}
 
-// CTA size of the one-CTA resampler, timed once per process for each
-// resampler and particle count (the sizes compute the same ancestors)
-static int one_cta_threads(bpf_handle* h, int resampler) {
+// The cluster size and threads of that resampler, timed once per process for
+// each device, resampler and particle count (all compute the same ancestors)
+static int one_filter_plan(bpf_handle* h, int resampler) {
   static std::mutex mu;
-  static std::map<std::pair<int, int>, int> tuned;
-  const std::pair<int, int> key(resampler, h->n);
+  static std::map<std::tuple<int, int, int>, bpf::ResamplePlan> tuned;
+  int dev = 0;
+  BPF_TRY(cudaGetDevice(&dev));
+  const std::tuple<int, int, int> key(dev, resampler, h->n);
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = tuned.find(key);
     if (it != tuned.end()) {
-      h->one_threads = it->second;
+      h->one_plan = it->second;
+      h->one_plan.order = h->one_order;
+      h->one_plan.sorted = h->one_filt;
       return BPF_OK;
     }
   }
-  int rc = bpf::tune_batch_resample(h->one_filt, h->one_order, 1, h->n, h->ld, h->stream, &h->one_threads, nullptr);
+  int rc = bpf::tune_batch_resample(h->one_filt, &h->one_plan, h->ld, h->stream, nullptr);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(mu);
-  tuned[key] = h->one_threads;
+  tuned[key] = h->one_plan;
   return BPF_OK;
 }
 
@@ -456,8 +463,8 @@ static int create_common(bpf_handle* h, const bpf_config* config, int dim, int p
     cudaGetLastError();
     h->host_stats = nullptr;  // read back through pageable memory instead
   }
-  if (h->n <= kOneCtaMaxParticles) {
-    // one CTA resamples the whole filter (the resampler reads n, off,
+  if (h->n <= cluster_max_particles(config->resampler)) {
+    // one cluster resamples the whole filter (the resampler reads n, off,
     // resampler, B and seed of the table entry)
     bpf::BatchFilter f{};
     f.n = h->n;
@@ -474,8 +481,10 @@ static int create_common(bpf_handle* h, const bpf_config* config, int dim, int p
       bpf_destroy(h);
       return BPF_E_NOMEM;
     }
-    rc = bpf::configure_batch_resample(h->n);
-    if (!rc) rc = one_cta_threads(h, config->resampler);
+    bpf::plan_batch_resample(&f, 1, &h->one_plan);
+    h->one_plan.order = h->one_order;
+    h->one_plan.sorted = h->one_filt;
+    rc = one_filter_plan(h, config->resampler);
     if (rc) { bpf_destroy(h); return rc; }
   } else if (config->resampler == BPF_RESAMPLER_SYSTEMATIC && bpf::autotuned_shape(h->n) == -1) {
     // the one-launch cooperative resampler's tile shape for this N, tuned
