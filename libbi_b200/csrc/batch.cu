@@ -96,6 +96,7 @@ k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld
                        const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
                        double* hist, int nf, int k) {
   __shared__ T sx[D][kL96Block];
+  pdl_wait();  // the resampler's ancestors and statistics
   const int f = __ldg(blk2f + blockIdx.x);
   const BatchFilter fd = filt[f];
   StepStats* st = stats + f;
@@ -123,6 +124,7 @@ k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld
     if (resampled) as[col] = src;
     lw_push(part, l);
   }
+  pdl_trigger();
   if (transition_reduce_tail(part, partials, blockIdx.x, fd.block0, fd.nblocks, counters + f, fd.n, st, ok,
                              resampled, y != nullptr))
     batch_record(st, hist, nf, f, k);
@@ -135,6 +137,7 @@ k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld,
                       const BatchFilter* __restrict__ filt, const PZParams* __restrict__ prms,
                       const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
                       double* hist, int nf, int k) {
+  pdl_wait();  // the resampler's ancestors and statistics
   const int f = __ldg(blk2f + blockIdx.x);
   const BatchFilter fd = filt[f];
   StepStats* st = stats + f;
@@ -157,6 +160,7 @@ k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld,
     if (resampled) as[col] = src;
     lw_push(part, l);
   }
+  pdl_trigger();
   if (transition_reduce_tail(part, partials, blockIdx.x, fd.block0, fd.nblocks, counters + f, fd.n, st, ok,
                              resampled, y != nullptr))
     batch_record(st, hist, nf, f, k);
@@ -184,9 +188,9 @@ int launch_batch_init(const ModelArgs& m, void* x, int ld, double* lw, const Bat
 
 #define BATCH_L96_CASE(TT, DD)                                                                              \
   case DD:                                                                                                  \
-    k_batch_l96_transition<TT, DD><<<blocks, kL96Block, 0, st>>>(                                           \
-        (const TT*)x_in, (TT*)x_out, ld, as, lw, (const TT*)y, t1, t2, step, filt, (const L96Params*)prms, \
-        blk2f, stats, partials, counters, hist, nf, k);                                                     \
+    BPF_TRY(launch_pdl(k_batch_l96_transition<TT, DD>, dim3(blocks), dim3(kL96Block), 0, st, (const TT*)x_in, \
+                       (TT*)x_out, ld, as, lw, (const TT*)y, t1, t2, step, filt, (const L96Params*)prms,     \
+                       blk2f, stats, partials, counters, hist, nf, k));                                       \
     break;
 
 int launch_batch_transition(const ModelArgs& m, const void* x_in, void* x_out, int ld, int* as, double* lw,
@@ -208,9 +212,9 @@ int launch_batch_transition(const ModelArgs& m, const void* x_in, void* x_out, i
       }
     }
   } else {
-    k_batch_pz_transition<double><<<blocks, kPZBlock, 0, st>>>(
-        (const double*)x_in, (double*)x_out, ld, as, lw, (const double*)y, t1, t2, step, filt,
-        (const PZParams*)prms, blk2f, stats, partials, counters, hist, nf, k);
+    BPF_TRY(launch_pdl(k_batch_pz_transition<double>, dim3(blocks), dim3(kPZBlock), 0, st, (const double*)x_in,
+                       (double*)x_out, ld, as, lw, (const double*)y, t1, t2, step, filt, (const PZParams*)prms,
+                       blk2f, stats, partials, counters, hist, nf, k));
   }
   BPF_TRY(cudaGetLastError());
   return BPF_OK;

@@ -187,7 +187,10 @@ k_batch_resample(const double* __restrict__ lw, int* __restrict__ as, const Batc
   __shared__ double s_W, s_yW;  // the weights' sum; its reciprocal, or its logarithm (multinomial)
   __shared__ int s_i[kGroup], s_z[kGroup], s_nbig, s_end;
   __shared__ int s_big[kBigMax][3];
-  pdl_trigger();  // a single filter's transition, a programmatic dependent, may be scheduled
+  // the transition after this kernel, a programmatic dependent, may be
+  // scheduled; this kernel is one of the transition before it
+  pdl_trigger();
+  pdl_wait();
   // the filter's entry and number, then its first log-weights and its gate:
   // two rounds of loads
   const BatchFilter fd = sorted[blockIdx.x / G];
@@ -460,7 +463,9 @@ static int launch_nt(const double* lw, int* as, const ResamplePlan& p, StepStats
   static unsigned configured = 0;
   BPF_TRY(set_dyn_smem_once(k_batch_resample<NT>, smem_bytes(BPF_BATCH_MAX_PARTICLES, kGroup, true), configured));
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)p.group;
   at[0].val.clusterDim.y = 1;
@@ -470,7 +475,7 @@ static int launch_nt(const double* lw, int* as, const ResamplePlan& p, StepStats
   cfg.dynamicSmemBytes = (size_t)smem_bytes(p.max_n, p.group, p.mult);
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   BPF_TRY(cudaLaunchKernelEx(&cfg, k_batch_resample<NT>, lw, as, p.sorted, p.order, stats, lu_buf, os_buf, step, p.group,
                              smem_slots(chunk_of(p.max_n, p.group))));
   return BPF_OK;

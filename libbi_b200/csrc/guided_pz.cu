@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_pz_net(PZNetArgs a) {
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();  // the step, which waits for this kernel's outputs
+  pdl_wait();     // the resampler's ancestors and statistics
   const uint32_t taddr = s_taddr;
   const uint32_t tg = taddr + (uint32_t)(128 * g);  // the group's accumulator
   const uint32_t trow = tg + ((uint32_t)((warp & 3) * 32) << 16);
@@ -276,6 +278,7 @@ k_batch_pz_guided(const double* __restrict__ x_in, double* __restrict__ x_out, i
                   const BatchFilter* __restrict__ filt, const PZParams* __restrict__ prms,
                   const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
                   double* hist, int nf, int k, const float2* __restrict__ O) {
+  pdl_wait();  // the network's outputs
   const int f = __ldg(blk2f + blockIdx.x);
   const BatchFilter fd = filt[f];
   StepStats* st = stats + f;
@@ -307,6 +310,7 @@ k_batch_pz_guided(const double* __restrict__ x_in, double* __restrict__ x_out, i
     if (resampled) as[col] = src;
     lw_push(part, l);
   }
+  pdl_trigger();
   if (transition_reduce_tail(part, partials, blockIdx.x, fd.block0, fd.nblocks, counters + f, fd.n, st, ok,
                              resampled, true))
     batch_record(st, hist, nf, f, k);
@@ -348,12 +352,10 @@ int launch_batch_pz_guided(ProposalNet& net, const BatchPZGuidedArgs& a, cudaStr
   // one CTA per SM (its 206 KB of shared memory and 512 TMEM columns)
   const int need = (a.blocks + kNetGroups - 1) / kNetGroups;
   const int grid = need < sms[dev] ? need : sms[dev];
-  k_pz_net<<<grid, kNetThreads, kNetSmem, st>>>(n);
-  BPF_TRY(cudaGetLastError());
-  k_batch_pz_guided<<<a.blocks, kPZBlock, 0, st>>>(a.x_in, a.x_out, a.ld, a.as, a.lw, a.y, a.t1, a.t2, a.step,
-                                                   a.filt, a.prms, a.blk2f, a.stats, a.partials, a.counters,
-                                                   a.hist, a.nf, a.k, a.O);
-  BPF_TRY(cudaGetLastError());
+  BPF_TRY(launch_pdl(k_pz_net, dim3(grid), dim3(kNetThreads), kNetSmem, st, n));
+  BPF_TRY(launch_pdl(k_batch_pz_guided, dim3(a.blocks), dim3(kPZBlock), 0, st, a.x_in, a.x_out, a.ld, a.as, a.lw, a.y,
+                     a.t1, a.t2, a.step, a.filt, a.prms, a.blk2f, a.stats, a.partials, a.counters, a.hist, a.nf, a.k,
+                     (const float2*)a.O));
   return BPF_OK;
 }
 
