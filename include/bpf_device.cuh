@@ -133,40 +133,61 @@ __device__ __forceinline__ LwPartial block_combine(LwPartial v) {
 
 enum FinalizeMode { kFinalizeReduce = 0, kFinalizeStep = 1, kFinalizeLogsumexp = 2 };
 
-// Called by every thread of the last block: combine partials[0..np) in a
-// fixed order and write the statistics.
-__device__ __forceinline__ void finalize_partials(const LwPartial* partials, int np, int n,
-                                                  StepStats* st, int mode, int observed) {
-  // each thread folds a fixed, strided subset of the partials (max first,
-  // then rescaled sums); loads are issued kBatch at a time so that the last
-  // block waits for a few memory round trips, not one per partial
-  constexpr int kBatch = 8;
-  const int nt = blockDim.x;
+// the statistics of n log-weights whose combined partial is v (one thread)
+__device__ __forceinline__ void write_stats(const LwPartial& v, int n, StepStats* st, int mode, int observed) {
+  st->mx = v.mx;
+  st->s1 = v.s1;
+  st->s2 = v.s2;
+  // ess_reduce: sum.first^2 / sum.second; lW = mx + log(sum.first) - log(n)
+  st->ess = v.s1 * v.s1 / v.s2;
+  st->lW = v.mx + log(v.s1) - log((double)n);
+  if (mode == kFinalizeLogsumexp) {
+    st->lW = v.mx + log(v.s1);
+  } else if (mode == kFinalizeStep) {
+    if (observed) {
+      // BootstrapPF::correct, share/src/bi/filter/BootstrapPF.hpp:176-179
+      st->inc = st->lW - st->ll;
+      st->ll = st->lW;
+      st->step += 1;
+      // Resampler::resample trigger, share/src/bi/resampler/Resampler.hpp:168
+      st->resample = st->ess < st->ess_rel * (double)n ? 1 : 0;
+    } else {
+      st->resample = 0;
+    }
+  }
+}
+
+// Thread vt's share of the fold of partials[0..np) by nt threads: a fixed,
+// strided subset (max first, then rescaled sums), loads issued B at a time so
+// that the last block waits for a few memory round trips, not one per
+// partial.
+template <int B>
+__device__ __forceinline__ LwPartial fold_partials_b(const LwPartial* partials, int np, int vt, int nt) {
   double m = -INFINITY;
-  for (int base = 0; base < np; base += nt * kBatch) {
-    double v[kBatch];
+  for (int base = 0; base < np; base += nt * B) {
+    double v[B];
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-      const int i = base + k * nt + threadIdx.x;
+    for (int k = 0; k < B; ++k) {
+      const int i = base + k * nt + vt;
       v[k] = i < np ? __ldcg(&partials[i].mx) : -INFINITY;
     }
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k) m = fmax(m, v[k]);
+    for (int k = 0; k < B; ++k) m = fmax(m, v[k]);
   }
   LwPartial v;
   v.mx = m; v.s1 = 0.0; v.s2 = 0.0;
   if (!isinf(m)) {
-    for (int base = 0; base < np; base += nt * kBatch) {
-      double pm[kBatch], p1[kBatch], p2[kBatch];
+    for (int base = 0; base < np; base += nt * B) {
+      double pm[B], p1[B], p2[B];
 #pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
-        const int i = base + k * nt + threadIdx.x;
+      for (int k = 0; k < B; ++k) {
+        const int i = base + k * nt + vt;
         pm[k] = i < np ? __ldcg(&partials[i].mx) : 0.0;
         p1[k] = i < np ? __ldcg(&partials[i].s1) : 0.0;
         p2[k] = i < np ? __ldcg(&partials[i].s2) : 0.0;
       }
 #pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
+      for (int k = 0; k < B; ++k) {
         if (p1[k] == 0.0) continue;
         const double f = exp(pm[k] - m);
         v.s1 += p1[k] * f;
@@ -174,28 +195,44 @@ __device__ __forceinline__ void finalize_partials(const LwPartial* partials, int
       }
     }
   }
-  v = block_combine(v);
-  if (threadIdx.x == 0) {
-    st->mx = v.mx;
-    st->s1 = v.s1;
-    st->s2 = v.s2;
-    // ess_reduce: sum.first^2 / sum.second; lW = mx + log(sum.first) - log(n)
-    st->ess = v.s1 * v.s1 / v.s2;
-    st->lW = v.mx + log(v.s1) - log((double)n);
-    if (mode == kFinalizeLogsumexp) {
-      st->lW = v.mx + log(v.s1);
-    } else if (mode == kFinalizeStep) {
-      if (observed) {
-        // BootstrapPF::correct, share/src/bi/filter/BootstrapPF.hpp:176-179
-        st->inc = st->lW - st->ll;
-        st->ll = st->lW;
-        st->step += 1;
-        // Resampler::resample trigger, share/src/bi/resampler/Resampler.hpp:168
-        st->resample = st->ess < st->ess_rel * (double)n ? 1 : 0;
-      } else {
-        st->resample = 0;
-      }
+  return v;
+}
+
+__device__ __forceinline__ LwPartial fold_partials(const LwPartial* partials, int np, int vt, int nt) {
+  // one partial per thread at most (f = exp(0) = 1): its share is the
+  // partial itself.  This code runs once per launch, so its length counts:
+  // every line of it is a miss in the instruction cache.
+  if (np <= nt) {
+    LwPartial v = lw_empty();
+    if (vt < np) {
+      v.mx = __ldcg(&partials[vt].mx);
+      v.s1 = __ldcg(&partials[vt].s1);
+      v.s2 = __ldcg(&partials[vt].s2);
+      if (isinf(v.mx)) { v.s1 = 0.0; v.s2 = 0.0; }
     }
+    return v;
+  }
+  return np <= 4 * nt ? fold_partials_b<4>(partials, np, vt, nt) : fold_partials_b<8>(partials, np, vt, nt);
+}
+
+// Called by every thread of the last block: combine partials[0..np) in a
+// fixed order and write the statistics.
+__device__ __forceinline__ void finalize_partials(const LwPartial* partials, int np, int n,
+                                                  StepStats* st, int mode, int observed) {
+  const LwPartial v = block_combine(fold_partials(partials, np, threadIdx.x, blockDim.x));
+  if (threadIdx.x == 0) write_stats(v, n, st, mode, observed);
+}
+
+// one thread, after the statistics of a step: whether it resampled, and its
+// entry in a whole-filter run's record
+__device__ __forceinline__ void record_step(StepStats* st, int resampled, bool observed) {
+  st->resampled = resampled;
+  double* h = st->hist;
+  const int k = st->step;
+  if (h && observed && k >= 1 && k <= st->hist_n) {
+    h[3 * (k - 1) + 0] = st->inc;
+    h[3 * (k - 1) + 1] = st->ess;
+    h[3 * (k - 1) + 2] = (double)resampled;
   }
 }
 
@@ -208,31 +245,32 @@ __device__ __forceinline__ void finalize_partials(const LwPartial* partials, int
 __device__ __forceinline__ bool transition_reduce_tail(LwPartial part, LwPartial* partials, int pidx, int pbase,
                                                        int np, unsigned* counter, int n, StepStats* st, bool ok,
                                                        int resampled, bool observed) {
-  part = block_combine(part);
-  if (threadIdx.x == 0) partials[pidx] = part;
+  // the block's own combination and the last block's share one copy of the
+  // code, so that the second finds it in the instruction cache
   __shared__ bool am_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = atomicAdd(counter, 1u) == (unsigned)np - 1;
-  __syncthreads();
-  if (am_last) {
-    __threadfence();
-    if (ok) {
-      finalize_partials(partials + pbase, np, n, st, kFinalizeStep, observed);
-      if (threadIdx.x == 0) {
-        st->resampled = resampled;
-        double* h = st->hist;
-        const int k = st->step;
-        if (h && observed && k >= 1 && k <= st->hist_n) {
-          h[3 * (k - 1) + 0] = st->inc;
-          h[3 * (k - 1) + 1] = st->ess;
-          h[3 * (k - 1) + 2] = (double)resampled;
-        }
-      }
+#pragma unroll 1
+  for (int pass = 0;; ++pass) {
+    part = block_combine(part);
+    if (pass == 1) break;
+    if (threadIdx.x == 0) {
+      partials[pidx] = part;
+      __threadfence();
+      am_last = atomicAdd(counter, 1u) == (unsigned)np - 1;
     }
-    if (threadIdx.x == 0) *counter = 0;
+    __syncthreads();
+    if (!am_last) return false;
+    __threadfence();
+    if (!ok) break;
+    part = fold_partials(partials + pbase, np, threadIdx.x, blockDim.x);
   }
-  return am_last;
+  if (threadIdx.x == 0) {
+    if (ok) {
+      write_stats(part, n, st, kFinalizeStep, observed);
+      record_step(st, resampled, observed);
+    }
+    *counter = 0;
+  }
+  return true;
 }
 
 

@@ -57,8 +57,7 @@ __global__ void k_batch_l96_init(T* x, int ld, int D, double* lw, const BatchFil
   for (int b = 0; b < (D + 3) / 4; ++b) {
     bpf_u32x4 r = bpf_draw(fd.seed, (uint32_t)p, 0u, (uint32_t)b, BPF_RNG_INIT);
     T z[4];
-    box_muller(r.v[0], r.v[1], z[0], z[1]);
-    box_muller(r.v[2], r.v[3], z[2], z[3]);
+    box_muller4(r, z);
     for (int j = 0; j < 4; ++j) {
       const int i = 4 * b + j;
       if (i < D) x[(size_t)i * ld + col] = Prec<T>::fma_(sd, z[j], mean);

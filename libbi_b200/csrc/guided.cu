@@ -236,8 +236,7 @@ __global__ void __launch_bounds__(kGTile * TILES, TILES == 1 ? 3 : 2) k_guided_f
           for (int h = 0; h < 2; ++h) {
             bpf_u32x4 rr = bpf_draw(seed, (uint32_t)p, (uint32_t)step, (uint32_t)(2 * c + h), BPF_RNG_NOISE);
             float z[4];
-            bpf_normal_pair_f(rr.v[0], rr.v[1], &z[0], &z[1]);
-            bpf_normal_pair_f(rr.v[2], rr.v[3], &z[2], &z[3]);
+            box_muller4(rr, z);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int q = 4 * h + j, i = 8 * c + q;

@@ -18,6 +18,7 @@
 #include "internal.cuh"
 #include "reduce.cuh"
 #include "../../include/bpf_math.h"
+#include "f32x2.cuh"
 
 #include <cmath>
 
@@ -50,6 +51,18 @@ __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, float& z0, fl
 }
 __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, double& z0, double& z1) {
   bpf_normal_pair_d(a, b, &z0, &z1);
+}
+
+// the four normals of a Philox block: two pairs, in FP32 side by side
+__device__ __forceinline__ void box_muller4(const bpf_u32x4& r, float (&z)[4]) {
+  pair::f2 z0, z1;
+  pair::normal_pair(r.v[0], r.v[1], r.v[2], r.v[3], z0, z1);
+  pair::unpack(z0, z[0], z[2]);
+  pair::unpack(z1, z[1], z[3]);
+}
+__device__ __forceinline__ void box_muller4(const bpf_u32x4& r, double (&z)[4]) {
+  box_muller(r.v[0], r.v[1], z[0], z[1]);
+  box_muller(r.v[2], r.v[3], z[2], z[3]);
 }
 
 struct L96Params {
@@ -134,8 +147,7 @@ __device__ __forceinline__ double l96_noise_obs_impl(const T (&sx)[D][kL96Block]
   for (int b = 0; b < (D + 3) / 4; ++b) {
     bpf_u32x4 r = bpf_draw(seed, prng, (uint32_t)step, (uint32_t)b, BPF_RNG_NOISE);
     T z[4];
-    box_muller(r.v[0], r.v[1], z[0], z[1]);
-    box_muller(r.v[2], r.v[3], z[2], z[3]);
+    box_muller4(r, z);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int i = 4 * b + j;
