@@ -17,9 +17,11 @@
 // s clamped to [kSMin, kSMax] (zero gradient outside).  One step: gather a
 // minibatch (indices from the counter-based stream, tag BPF_RNG_DATA),
 // three dense layers forward, the loss gradient, five dense layers backward
-// (weight gradients are dense layers over the batch dimension; the operands
-// are read transposed through strides), bias gradients by column sums, and
-// an Adam update that also refreshes the BF16 weight copies.
+// (weight gradients are dense layers over the batch dimension), bias
+// gradients by column sums, and an Adam update that also refreshes the BF16
+// weight copies: two launches for the Lorenz-96 network (train.cu), layer by
+// layer here for the small PZ network (operands read transposed through
+// strides).
 #include "internal.cuh"
 #include "model_body.cuh"
 #include "mlp.cuh"
@@ -46,23 +48,6 @@ __global__ void k_rk4_mean(const float* __restrict__ x, float* __restrict__ m, i
   l96_rk4<float, D>(v, 0.0, dt, (float)F, (float)h);
 #pragma unroll
   for (int i = 0; i < D; ++i) m[(size_t)p * D + i] = v[i];
-}
-
-// minibatch row b <- dataset row idx(b): standardised input [x_t, y - m]
-// (BF16) and the regression target r0 = x_{t+1} - m(x_t)
-__global__ void k_gather_batch(const float* __restrict__ xt, const float* __restrict__ mt,
-                               const float* __restrict__ xt1, const float* __restrict__ yt1, int n, int D, int B,
-                               uint64_t seed, int step, const float* __restrict__ shift,
-                               const float* __restrict__ scale, __nv_bfloat16* U, float* r0) {
-  const int b = blockIdx.x;
-  if (b >= B) return;
-  bpf_u32x4 w = bpf_draw(seed, (uint32_t)b, (uint32_t)step, 0u, BPF_RNG_DATA);
-  const size_t row = (size_t)(((uint64_t)w.v[0] << 32 | w.v[1]) % (uint64_t)n);
-  for (int j = threadIdx.x; j < 2 * D; j += blockDim.x) {
-    const float v = j < D ? xt[row * D + j] : yt1[row * D + (j - D)] - mt[row * D + (j - D)];
-    U[(size_t)b * 2 * D + j] = __float2bfloat16((v - shift[j]) * scale[j]);
-  }
-  for (int i = threadIdx.x; i < D; i += blockDim.x) r0[(size_t)b * D + i] = xt1[row * D + i] - mt[row * D + i];
 }
 
 // PZ training rows from states x_t (n x 2, FP64): the transition's log-noise
@@ -292,6 +277,13 @@ int proposal_forward(ProposalNet& p, const __nv_bfloat16* U, int B, __nv_bfloat1
 }
 
 static int loss_and_grad(ProposalNet& p, int B, cudaStream_t st) {
+  if (p.l96) {
+    TrainBatch t;
+    t.B = B;
+    int rc = launch_train_tile(p, t, st);
+    if (!rc) rc = launch_reduce_adam(p, B, p.loss, false, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 1.0f, st);
+    return rc;
+  }
   const int din = p.din, H = p.hidden, dout = p.dout, D = p.dim;
   int rc = proposal_forward(p, p.U, B, p.H1, p.H2, p.O, st);
   if (rc) return rc;
@@ -338,6 +330,7 @@ int ProposalNet::alloc(int d, int hid, int cap_batch, int din_) {
   nparams = o_b3 + dout;
   k1 = (din + 15) / 16 * 16;
   pz = din == 3 && dout == 2 && hidden == kProposalHidden;
+  l96 = din == 80 && dout == 80 && hidden == kProposalHidden;
   pk_w1 = 0;
   if (pz) {
     pk_w2 = pk_w1 + hidden * kPZNetK1 * 2;
@@ -363,13 +356,22 @@ int ProposalNet::alloc(int d, int hid, int cap_batch, int din_) {
   if (!rc) rc = A((void**)&err, sizeof(int));
   if (!rc) rc = A((void**)&loss, sizeof(double));
   if (!rc) rc = A((void**)&U, (size_t)cap * din * 2);
+  if (!rc) rc = A((void**)&r0, (size_t)cap * dim * 4);
+  if (l96) {
+    // the shares of the weight gradients, the bias sums and the losses
+    ws_floats = (long long)kTrainMaxShares * nparams;
+    if (!rc) rc = A((void**)&ws, (size_t)ws_floats * 4);
+    if (!rc) rc = A((void**)&colpart, (size_t)train_colpart_floats(cap) * 4);
+    if (!rc) rc = A((void**)&loss_part, (size_t)((cap + 127) / 128) * sizeof(double));
+    if (rc) cudaGetLastError();
+    return rc;
+  }
   if (!rc) rc = A((void**)&H1, (size_t)cap * hidden * 2);
   if (!rc) rc = A((void**)&H2, (size_t)cap * hidden * 2);
   if (!rc) rc = A((void**)&O, (size_t)cap * dout * 4);
   if (!rc) rc = A((void**)&dO, (size_t)cap * dout * 2);
   if (!rc) rc = A((void**)&dH, (size_t)cap * hidden * 4);
   if (!rc) rc = A((void**)&dZ, (size_t)cap * hidden * 2);
-  if (!rc) rc = A((void**)&r0, (size_t)cap * dim * 4);
   if (!rc) rc = A((void**)&colpart, (size_t)((cap + kColChunk - 1) / kColChunk) * (hidden > dout ? hidden : dout) * 4);
   if (!rc) rc = A((void**)&loss_part, (size_t)((cap + 255) / 256) * sizeof(double));
   // room for one partial product per SM of the widest weight gradient
@@ -381,7 +383,7 @@ int ProposalNet::alloc(int d, int hid, int cap_batch, int din_) {
 
 void ProposalNet::release() {
   void* ps[] = {params, params_h, packed, grads, m1, m2, shift, scale, err, loss, U, H1, H2, O, dO, dH, dZ, r0, mt,
-                 colpart, loss_part, ws, feat, target};
+                 colpart, loss_part, losses, ws, feat, target};
   for (void* q : ps)
     if (q) cudaFree(q);
 }
@@ -574,33 +576,61 @@ int bpf_proposal_train(bpf_proposal* q, int steps, int batch, double lr, float* 
   // learning rate: linear warm-up over the first 5% of the steps, then a
   // cosine decay to a tenth
   const int warm = steps / 20 > 1 ? steps / 20 : 1;
+  // the steps' losses stay on the device until the last one is enqueued
+  if (steps > p.losses_cap) {
+    if (p.losses) cudaFree(p.losses);
+    p.losses = nullptr;
+    p.losses_cap = 0;
+    if (cudaMalloc((void**)&p.losses, (size_t)steps * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();
+      return BPF_E_NOMEM;
+    }
+    p.losses_cap = steps;
+  }
   for (int s = 0; s < steps; ++s) {
     const double w = s < warm ? (double)(s + 1) / warm : 1.0;
     const double c = 0.1 + 0.9 * 0.5 * (1.0 + std::cos(3.14159265358979323846 * s / (double)steps));
     const double lr_s = lr * w * c;
-    if (p.feat)
+    int rc = BPF_OK;
+    if (p.l96) {
+      bpf::TrainBatch t;
+      t.xt = q->xt;
+      t.xt1 = q->xt1;
+      t.yt1 = q->yt1;
+      t.n = q->n;
+      t.step = q->train_step;
+      t.B = batch;
+      t.seed = q->seed;
+      rc = bpf::launch_train_tile(p, t, q->stream);
+    } else {
       bpf::k_gather_rows<<<batch, 128, 0, q->stream>>>(p.feat, p.target, p.rows, p.din, p.dim, batch, q->seed,
                                                        q->train_step, p.shift, p.scale, p.U, p.r0);
-    else
-      bpf::k_gather_batch<<<batch, 128, 0, q->stream>>>(q->xt, p.mt, q->xt1, q->yt1, q->n, p.dim, batch, q->seed,
-                                                        q->train_step, p.shift, p.scale, p.U, p.r0);
-    int rc = bpf::loss_and_grad(p, batch, q->stream);
+      rc = bpf::loss_and_grad(p, batch, q->stream);
+    }
     if (rc) return rc;
     ++q->adam_step;
     ++q->train_step;
     const float c1 = 1.0f - std::pow(b1, (float)q->adam_step), c2 = 1.0f - std::pow(b2, (float)q->adam_step);
-    bpf::k_adam<<<(p.nparams + 255) / 256, 256, 0, q->stream>>>(p.params, p.grads, p.m1, p.m2, p.params_h,
-                                                               p.nparams, (float)lr_s, b1, b2, eps, c1, c2);
-    BPF_TRY(cudaGetLastError());
-    if (loss_trace) {
-      double l = 0.0;
-      BPF_TRY(cudaMemcpyAsync(&l, p.loss, sizeof(double), cudaMemcpyDeviceToHost, q->stream));
-      BPF_TRY(cudaStreamSynchronize(q->stream));
-      loss_trace[s] = (float)l;
+    if (p.l96) {
+      rc = bpf::launch_reduce_adam(p, batch, p.losses + s, true, (float)lr_s, b1, b2, eps, c1, c2, q->stream);
+      if (rc) return rc;
+    } else {
+      bpf::k_adam<<<(p.nparams + 255) / 256, 256, 0, q->stream>>>(p.params, p.grads, p.m1, p.m2, p.params_h,
+                                                                 p.nparams, (float)lr_s, b1, b2, eps, c1, c2);
+      BPF_TRY(cudaGetLastError());
+      BPF_TRY(cudaMemcpyAsync(p.losses + s, p.loss, sizeof(double), cudaMemcpyDeviceToDevice, q->stream));
     }
   }
-  int rc = bpf::pack_weights(p, q->stream);
-  if (rc) return rc;
+  if (loss_trace && steps > 0) {
+    std::vector<double> l((size_t)steps);
+    BPF_TRY(cudaMemcpyAsync(l.data(), p.losses, l.size() * sizeof(double), cudaMemcpyDeviceToHost, q->stream));
+    BPF_TRY(cudaStreamSynchronize(q->stream));
+    for (int s = 0; s < steps; ++s) loss_trace[s] = (float)l[s];
+  }
+  if (!p.l96) {  // the two-launch step keeps the images current
+    const int rc = bpf::pack_weights(p, q->stream);
+    if (rc) return rc;
+  }
   return check_err(q);
 }
 

@@ -25,6 +25,8 @@ struct ProposalNet {
   // PZ network (din 3, dout 2): the images hold the biases of layers 1 and 2
   // as extra K columns (kPZNetK1, kPZNetK2) and W3 padded to 16 rows
   bool pz = false;
+  // L96 network (din 80, dout 80): trained by the two-launch step (train.cu)
+  bool l96 = false;
   // parameter vector: W1 [hidden x din], b1, W2 [hidden x hidden], b2,
   // W3 [dout x hidden], b3 (offsets in floats)
   int o_w1 = 0, o_b1 = 0, o_w2 = 0, o_b2 = 0, o_w3 = 0, o_b3 = 0, nparams = 0;
@@ -46,14 +48,16 @@ struct ProposalNet {
   int rows = 0;
   // the BF16 weight matrices as shared-memory images in the canonical
   // K-major layout (tc.cuh): W1 at byte pk_w1, W2 at pk_w2, W3 at pk_w3;
-  // rebuilt by pack_weights whenever params_h changes outside training and
-  // at the end of every training call
+  // rebuilt by pack_weights whenever params_h changes outside training and at
+  // the end of a PZ training call; the L96 training step keeps them current
   unsigned char* packed = nullptr;
   int pk_w1 = 0, pk_w2 = 0, pk_w3 = 0, pk_bytes = 0;
-  float* colpart = nullptr;  // per-chunk column sums of the bias gradients
-  float* ws = nullptr;       // split-K workspace of the weight-gradient layers
+  float* colpart = nullptr;  // per-chunk column sums of the bias gradients (L96: all three layers')
+  float* ws = nullptr;       // shares (L96: per tile) or split-K parts of the weight gradients
   long long ws_floats = 0;
   double* loss_part = nullptr;  // per-block loss sums
+  double* losses = nullptr;     // losses of a training call's steps
+  int losses_cap = 0;
 
   const __nv_bfloat16* w1h() const { return params_h + o_w1; }
   const __nv_bfloat16* w2h() const { return params_h + o_w2; }
@@ -72,6 +76,24 @@ int pack_weights(ProposalNet& p, cudaStream_t st);
 // O [B x dout] = MLP(U [B x din]); H1, H2 [B x hidden] hold the activations
 int proposal_forward(ProposalNet& p, const __nv_bfloat16* U, int B, __nv_bfloat16* H1, __nv_bfloat16* H2, float* O,
                      cudaStream_t st);
+
+// The training step of the L96 network in two launches (train.cu).
+// A minibatch of B rows: drawn from the data set (xt, ProposalNet::mt, xt1,
+// yt1, n rows) with the draws of `step`, or (xt null) given in
+// ProposalNet::U and r0.
+struct TrainBatch {
+  const float *xt = nullptr, *xt1 = nullptr, *yt1 = nullptr;
+  int n = 0, step = 0, B = 0;
+  uint64_t seed = 0;
+};
+// CTAs, and so shares of the weight gradients, at most: one per SM
+constexpr int kTrainMaxShares = 148;
+long long train_colpart_floats(int cap);
+int launch_train_tile(ProposalNet& p, const TrainBatch& t, cudaStream_t st);
+// the gradient into ProposalNet::grads, the mean loss to *loss (device), and
+// with `update` an Adam step of the parameters, their BF16 copy and images
+int launch_reduce_adam(ProposalNet& p, int B, double* loss, bool update, float lr, float b1, float b2, float eps,
+                       float c1, float c2, cudaStream_t st);
 
 // one guided filter step (guided.cu)
 struct GuidedArgs {
