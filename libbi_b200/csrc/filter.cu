@@ -99,6 +99,7 @@ struct bpf_resampler {
   int shape = -1;  // pinned tile shape of the one-launch systematic kernel
   cudaStream_t stream = nullptr;
   bpf::ResampleScratch rs;
+  bpf::StepStats* host_stats = nullptr;  // pinned copy of the statistics
   // optional device timing of the compute kernels of each call (events
   // after the status reset and before the read-back)
   bool timing = false;
@@ -1054,6 +1055,10 @@ int bpf_resampler_create(int kind, int max_n, int metropolis_steps, void* stream
   r->stream = (cudaStream_t)stream;
   int rc = bpf::scratch_alloc(r->rs, max_n);
   if (rc) { delete r; return rc; }
+  if (cudaMallocHost((void**)&r->host_stats, sizeof(bpf::StepStats)) != cudaSuccess) {
+    cudaGetLastError();
+    r->host_stats = nullptr;  // read back through pageable memory instead
+  }
   *out = r;
   return BPF_OK;
 }
@@ -1063,6 +1068,7 @@ int bpf_resampler_destroy(bpf_resampler* r) {
   if (r->stream) cudaStreamSynchronize(r->stream); else cudaDeviceSynchronize();
   for (cudaEvent_t e : r->ev)
     if (e) cudaEventDestroy(e);
+  if (r->host_stats) cudaFreeHost(r->host_stats);
   bpf::scratch_free(r->rs);
   delete r;
   return BPF_OK;
@@ -1095,8 +1101,11 @@ static int timing_collect(bpf_resampler* r) {
 }
 
 static int read_rs_stats(bpf_resampler* r, bpf::StepStats* s) {
-  BPF_TRY(cudaMemcpyAsync(s, r->rs.stats, sizeof(*s), cudaMemcpyDeviceToHost, r->stream));
+  // through the handle's pinned copy: a direct DMA instead of a staged copy
+  bpf::StepStats* dst = r->host_stats ? r->host_stats : s;
+  BPF_TRY(cudaMemcpyAsync(dst, r->rs.stats, sizeof(*s), cudaMemcpyDeviceToHost, r->stream));
   BPF_TRY(cudaStreamSynchronize(r->stream));
+  if (dst != s) *s = *dst;
   return timing_collect(r);
 }
 
@@ -1138,9 +1147,8 @@ int bpf_resampler_set_shape(bpf_resampler* r, int shape) {
 
 int bpf_ess_reduce(bpf_resampler* r, const double* lw, int n, double* lW, double* ess) {
   if (!r || !lw || n <= 0 || n > r->rs.max_n) return BPF_E_INVALID;
-  int rc = reset_status(r);
+  int rc = timing_begin(r);
   if (rc) return rc;
-  if ((rc = timing_begin(r))) return rc;
   rc = bpf::launch_lw_reduce(lw, n, r->rs, r->stream);
   if (rc) return rc;
   if ((rc = timing_end(r))) return rc;
@@ -1154,9 +1162,8 @@ int bpf_ess_reduce(bpf_resampler* r, const double* lw, int n, double* lW, double
 
 int bpf_logsumexp_reduce(bpf_resampler* r, const double* lw, int n, double* out) {
   if (!r || !lw || n <= 0 || n > r->rs.max_n) return BPF_E_INVALID;
-  int rc = reset_status(r);
+  int rc = timing_begin(r);
   if (rc) return rc;
-  if ((rc = timing_begin(r))) return rc;
   rc = bpf::launch_logsumexp(lw, n, r->rs, r->stream);
   if (rc) return rc;
   if ((rc = timing_end(r))) return rc;
@@ -1170,7 +1177,8 @@ int bpf_logsumexp_reduce(bpf_resampler* r, const double* lw, int n, double* out)
 int bpf_resampler_ancestors(bpf_resampler* r, const double* lw, int n, const double* uniforms, int permute,
                             int* as, int* Os) {
   if (!r || !lw || !as || n <= 0 || n > r->rs.max_n) return BPF_E_INVALID;
-  int rc = reset_status(r);
+  // the scan resamplers' first pass resets the status (k_lw_max)
+  int rc = r->kind == BPF_RESAMPLER_METROPOLIS ? reset_status(r) : BPF_OK;
   if (rc) return rc;
   bpf::ResampleArgs ra;
   ra.kind = r->kind;

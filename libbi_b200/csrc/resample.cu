@@ -142,9 +142,123 @@ __device__ __forceinline__ int block_max_int(int v) {
   return r;
 }
 
+// The first index whose entry of the nondecreasing A[0..n) exceeds x (n if
+// none does), by a whole warp: 32 probes at a time, so that 2^20 entries take
+// four round trips instead of twenty.
+template <class T>
+__device__ __forceinline__ int warp_upper_bound(const T* __restrict__ A, int n, T x) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int step = (hi - lo + 31) >> 5;
+    const int i = lo + lane * step;
+    const unsigned above = __ballot_sync(0xffffffffu, i < hi && __ldg(A + i) > x);
+    // probes inside [lo, hi) that are not above x form a prefix of the lanes
+    const int probes = (hi - lo + step - 1) / step;
+    const int first = above ? __ffs(above) - 1 : probes;
+    if (first < probes) hi = lo + first * step;
+    if (first > 0) lo = lo + (first - 1) * step + 1;
+  }
+  return lo;
+}
+
+// The same for one x per thread, nondecreasing over the block's threads from
+// x_first to x_last: two warps bracket the block's answers, then each thread
+// searches between them (a few steps in lines its neighbours read too,
+// instead of log2 n dependent loads).
+template <class T>
+__device__ __forceinline__ void block_bounds(const T* __restrict__ A, int n, T x_first, T x_last, int (&bound)[2]) {
+  __shared__ int s_bound[2];
+  const int warp = threadIdx.x >> 5;
+  __syncthreads();  // an earlier call's bounds have been read
+  if (warp < 2) {
+    const int r = warp_upper_bound(A, n, warp == 0 ? x_first : x_last);
+    if ((threadIdx.x & 31) == 0) s_bound[warp] = r;
+  }
+  __syncthreads();
+  bound[0] = s_bound[0];
+  bound[1] = s_bound[1];
+}
+
+template <class T>
+__device__ __forceinline__ int upper_bound_in(const T* __restrict__ A, int lo, int hi, T x) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(A + mid) > x) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+
+template <class T>
+__device__ __forceinline__ int block_upper_bound(const T* __restrict__ A, int n, T x, T x_first, T x_last) {
+  int bound[2];
+  block_bounds(A, n, x_first, x_last, bound);
+  return upper_bound_in(A, bound[0], bound[1], x);
+}
+
 __device__ __forceinline__ bool gate_closed(const int* gate, const StepStats* st) {
   if (gate != nullptr && *gate == 0) return true;
   return st->status != BPF_OK;
+}
+
+// ---------------------------------------------------------------------------
+// The first pass of a stand-alone call: the largest log-weight (NaN ignored),
+// which is all the resamplers need of the statistics, and a clean start for
+// the rest of the call (status, grid-barrier words, the one-launch kernel's
+// epoch).  8 bytes per log-weight and two operations, against the full
+// reduction's exp (k_lw_reduce: 17 us at 4 M log-weights in L2).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kBlock)
+k_lw_max(const double* __restrict__ lw, int n, LwPartial* partials, StepStats* st, unsigned* counters) {
+  constexpr int K = 8;
+  double m = -INFINITY;
+  const long long stride = (long long)gridDim.x * kBlock * K;
+  long long i = (long long)(blockIdx.x * kBlock + threadIdx.x) * 2;
+  if ((reinterpret_cast<uintptr_t>(lw) & 15) == 0) {
+    // consecutive threads on consecutive pairs, K / 2 pairs in flight
+    const long long row = (long long)gridDim.x * kBlock * 2;
+    for (; i + (K / 2 - 1) * row + 1 < n; i += stride) {
+      double2 v[K / 2];
+#pragma unroll
+      for (int k = 0; k < K / 2; ++k) v[k] = __ldg(reinterpret_cast<const double2*>(lw + i + k * row));
+#pragma unroll
+      for (int k = 0; k < K / 2; ++k) m = fmax(m, fmax(v[k].x, v[k].y));
+    }
+    for (; i < n; i += row) {
+      m = fmax(m, __ldg(lw + i));
+      if (i + 1 < n) m = fmax(m, __ldg(lw + i + 1));
+    }
+  } else {
+    for (i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) m = fmax(m, __ldg(lw + i));
+  }
+  __shared__ double s_m[kBlock / 32];
+  __shared__ bool am_last;
+#pragma unroll 1
+  for (int pass = 0;; ++pass) {
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = warp_max((threadIdx.x & 31) < kBlock / 32 ? s_m[threadIdx.x & 31] : -INFINITY);
+    if (pass == 1) break;
+    if (threadIdx.x == 0) {
+      partials[blockIdx.x].mx = m;
+      __threadfence();
+      am_last = atomicAdd(counters + 3, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!am_last) return;
+    __threadfence();
+    m = -INFINITY;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kBlock) m = fmax(m, __ldcg(&partials[b].mx));
+  }
+  if (threadIdx.x == 0) {
+    st->mx = m;
+    st->status = BPF_OK;
+    counters[3] = 0u;
+    counters[8] = 0u;
+    counters[9] = 0u;
+    counters[kEpochWord] += 1u;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -154,7 +268,7 @@ __global__ void __launch_bounds__(kBlock)
 k_weight_tile_sums(const double* __restrict__ lw, int n, StepStats* st,
                    u128* tile_sum, u128* tile_prefix,
                    int with_spacings, const double* u, uint64_t seed, int step,
-                   u128* vtile_sum, u128* vtile_prefix,
+                   u128* vtile_sum, u128* vtile_prefix, unsigned long long* qbuf, double* spbuf,
                    unsigned* counter, const int* gate) {
   if (gate_closed(gate, st)) return;
   const double mx = st->mx;
@@ -169,7 +283,14 @@ k_weight_tile_sums(const double* __restrict__ lw, int n, StepStats* st,
       double w = nanexp(__dsub_rn(v[k], mx));
       u128 q; q.lo = weight_to_fixed(w); q.hi = 0;
       acc = u128_add(acc, q);
-      if (with_spacings) vacc = u128_add(vacc, spacing_to_fixed(multinomial_spacing(u, i0 + k, n, seed, step)));
+      if (with_spacings) {
+        // kept for k_multinomial_prepare: 16 bytes against an exp, a draw, a
+        // logarithm and a division
+        const double sp = multinomial_spacing(u, i0 + k, n, seed, step);
+        vacc = u128_add(vacc, spacing_to_fixed(sp));
+        qbuf[i0 + k] = q.lo;
+        spbuf[i0 + k] = sp;
+      }
     }
   }
   u128 tot;
@@ -970,6 +1091,7 @@ k_offspring_from(const int* __restrict__ src, int n, int mode, const StepStats* 
   const int T = gridDim.x;
   const int i0 = t * kTile + threadIdx.x * kItems;
   int os[kItems];
+  int first_bound = 0;  // mode 1: the cumulative offspring before the tile
   if (mode == 0) {
     int v[kItems];
     int loc = 0;
@@ -980,15 +1102,11 @@ k_offspring_from(const int* __restrict__ src, int n, int mode, const StepStats* 
 #pragma unroll
     for (int k = 0; k < kItems; ++k) { run += v[k]; os[k] = run; }
   } else {
+    int bound[2];
+    block_bounds(src, n, t * kTile - 1, (t + 1) * kTile - 1, bound);
+    first_bound = bound[0];
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      int key = i0 + k, lo = 0, hi = n;
-      while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (__ldg(src + mid) <= key) lo = mid + 1; else hi = mid;
-      }
-      os[k] = lo;
-    }
+    for (int k = 0; k < kItems; ++k) os[k] = upper_bound_in(src, bound[0], bound[1], i0 + k);
   }
   s_last[threadIdx.x] = os[kItems - 1];
   __syncthreads();
@@ -1000,12 +1118,7 @@ k_offspring_from(const int* __restrict__ src, int n, int mode, const StepStats* 
   } else if (mode == 0) {
     prev = iprefix[t];
   } else {
-    int key = i0 - 1, lo = 0, hi = n;
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (__ldg(src + mid) <= key) lo = mid + 1; else hi = mid;
-    }
-    prev = lo;
+    prev = first_bound;
   }
   int zeros = 0;
 #pragma unroll
@@ -1034,8 +1147,8 @@ k_offspring_from(const int* __restrict__ src, int n, int mode, const StepStats* 
 // the ancestor a with E_a <= r < E_{a+1}.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock)
-k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* as, int* E, int* ecoarse,
-                    int coarse_shift, int* slot, const StepStats* st, const int* gate) {
+k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* as, int* E, int* slot,
+                    const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
   const int t = blockIdx.x;
   const int i0 = t * kTile + threadIdx.x * kItems;
@@ -1058,7 +1171,6 @@ k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* 
     if (i < n) {
       const int e = before - i + Z;
       E[i] = e;
-      if ((i & ((1 << coarse_shift) - 1)) == 0) ecoarse[i >> coarse_shift] = e;  // coarse search index
       if (z[k]) slot[Z] = i;
       else as[i] = i;
     }
@@ -1066,35 +1178,19 @@ k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* 
   }
 }
 
-// Childless slot of rank r receives the ancestor a with E_a <= r < E_{a+1}:
-// a search over every 2^coarse_shift-th value of E (held in shared memory),
-// then within that short segment.  One thread per rank, so the work is
-// balanced however the copies are distributed.
-constexpr int kMaxCoarse = 12288;  // 48 KB of coarse index
-
+// Childless slot of rank r receives the ancestor a with E_a <= r < E_{a+1}.
+// One thread per rank, so the work is balanced however the copies are
+// distributed.
 __global__ void __launch_bounds__(kBlock)
-k_permute_fill(int* as, const int* __restrict__ E, const int* __restrict__ ecoarse, int coarse_shift,
-               const int* __restrict__ slot, const int* zprefix, int n, int T, const StepStats* st,
-               const int* gate) {
+k_permute_fill(int* as, const int* __restrict__ E, const int* __restrict__ slot, const int* zprefix, int n, int T,
+               const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
-  extern __shared__ int s_coarse[];
-  const int nc = ((n - 1) >> coarse_shift) + 1;
-  for (int i = threadIdx.x; i < nc; i += blockDim.x) s_coarse[i] = ecoarse[i];
-  __syncthreads();
   const int R = zprefix[T];
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    int clo = 0, chi = nc;  // last segment whose first value is <= r (E[0] = 0 <= r)
-    while (clo < chi) {
-      int mid = (clo + chi) >> 1;
-      if (s_coarse[mid] <= r) clo = mid + 1; else chi = mid;
-    }
-    int lo = (clo - 1) << coarse_shift;
-    int hi = min(n, lo + (1 << coarse_shift));
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (__ldg(E + mid) <= r) lo = mid + 1; else hi = mid;
-    }
-    as[__ldg(slot + r)] = lo - 1;
+  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < R; b0 += (long long)gridDim.x * kBlock) {
+    const int base = (int)b0;
+    const int r = (int)min(b0 + threadIdx.x, (long long)R - 1);
+    const int a = block_upper_bound(E, n, r, base, (int)min(b0 + kBlock, (long long)R) - 1) - 1;
+    as[__ldg(slot + r)] = a;
   }
 }
 
@@ -1103,13 +1199,11 @@ k_permute_fill(int* as, const int* __restrict__ E, const int* __restrict__ ecoar
 __global__ void __launch_bounds__(kBlock)
 k_ancestors_from_Os(const int* __restrict__ Os, int n, int* as, const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (__ldg(Os + mid) <= j) lo = mid + 1; else hi = mid;
-    }
-    as[j] = lo < n ? lo : n - 1;  // Os[n-1] == n for valid offsets; bounds any other
+  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < n; b0 += (long long)gridDim.x * kBlock) {
+    const int base = (int)b0;
+    const int j = (int)min(b0 + threadIdx.x, (long long)n - 1);
+    const int r = block_upper_bound(Os, n, j, base, (int)min(b0 + kBlock, (long long)n) - 1);
+    as[j] = r < n ? r : n - 1;  // Os[n-1] == n for valid offsets; bounds any other
   }
 }
 
@@ -1119,28 +1213,25 @@ k_ancestors_from_Os(const int* __restrict__ Os, int n, int* as, const StepStats*
 // with one host thread: slot s gets the number of m with log(Ws_m) <= lu_s,
 // lu_s = log(W) + lMax_s, lMax_s = sum_{i > s} log(u)/i.
 // ---------------------------------------------------------------------------
+// Ws: the fixed-point weights in, the logarithms of the cumulative weights
+// out; lu: the spacings in, the log uniforms out (each thread's own entries).
 __global__ void __launch_bounds__(kBlock)
-k_multinomial_prepare(const double* __restrict__ lw, int n, StepStats* st,
-                      const u128* tile_prefix, const u128* vtile_prefix,
-                      const double* u, uint64_t seed, int step,
-                      double* Ws, double* lu, const int* gate) {
+k_multinomial_prepare(int n, const StepStats* st, const u128* tile_prefix, const u128* vtile_prefix, double* Ws,
+                      double* lu, const int* gate) {
   if (gate_closed(gate, st)) return;
-  const double mx = st->mx;
   const int t = blockIdx.x;
   const int T = gridDim.x;
   const int i0 = t * kTile + threadIdx.x * kItems;
   const double lW = log(u128_to_weight(tile_prefix[T]));
   const u128 Vtot = vtile_prefix[T];
-  double v[kItems];
-  load_blocked(lw, i0, n, v);
   unsigned long long q[kItems];
   u128 vv[kItems];
   u128 loc = u128_zero(), vloc = u128_zero();
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
-    bool in = i0 + k < n;
-    q[k] = in ? weight_to_fixed(nanexp(__dsub_rn(v[k], mx))) : 0ull;
-    vv[k] = in ? spacing_to_fixed(multinomial_spacing(u, i0 + k, n, seed, step)) : u128_zero();
+    const bool in = i0 + k < n;
+    q[k] = in ? reinterpret_cast<const unsigned long long*>(Ws)[i0 + k] : 0ull;
+    vv[k] = in ? spacing_to_fixed(lu[i0 + k]) : u128_zero();
     u128 qq; qq.lo = q[k]; qq.hi = 0;
     loc = u128_add(loc, qq);
     vloc = u128_add(vloc, vv[k]);
@@ -1153,7 +1244,7 @@ k_multinomial_prepare(const double* __restrict__ lw, int n, StepStats* st,
     u128 qq; qq.lo = q[k]; qq.hi = 0;
     Q = u128_add(Q, qq);
     if (i0 + k < n) {
-      Ws[i0 + k] = u128_to_weight(Q);
+      Ws[i0 + k] = log(u128_to_weight(Q));
       // suffix sum over slots >= s of the spacings, then lu = lW + lMax
       double lmax = -fixed_to_spacing(u128_sub(Vtot, V));
       lu[i0 + k] = __dadd_rn(lW, lmax);
@@ -1163,18 +1254,15 @@ k_multinomial_prepare(const double* __restrict__ lw, int n, StepStats* st,
 }
 
 __global__ void __launch_bounds__(kBlock)
-k_multinomial_search(const double* __restrict__ Ws, const double* __restrict__ lu, int n, int* as,
+k_multinomial_search(const double* __restrict__ lWs, const double* __restrict__ lu, int n, int* as,
                      const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-    const double x = lu[s];
-    int lo = 0, hi = n;
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (log(__ldg(Ws + mid)) <= x) lo = mid + 1; else hi = mid;
-    }
+  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < n; b0 += (long long)gridDim.x * kBlock) {
+    const int base = (int)b0;
+    const int s = (int)min(b0 + threadIdx.x, (long long)n - 1);
+    const int r = block_upper_bound(lWs, n, lu[s], lu[base], lu[(int)min(b0 + kBlock, (long long)n) - 1]);
     // the reference's loop can leave j = n when lu rounds up to log(W); clamp
-    as[s] = lo < n ? lo : n - 1;
+    as[s] = r < n ? r : n - 1;
   }
 }
 
@@ -1280,13 +1368,13 @@ void scratch_free(ResampleScratch& s) {
 
 // coarse index stride: the smallest power of two >= 16 that keeps the index
 // within max_entries entries
-static inline int coarse_shift(int n, int max_entries = kMaxCoarse) {
+static inline int coarse_shift(int n, int max_entries) {
   int sh = 4;
   while ((((long long)n + (1ll << sh) - 1) >> sh) > max_entries) ++sh;
   return sh;
 }
 
-static inline size_t fill_smem(int n, int max_entries = kMaxCoarse) {
+static inline size_t fill_smem(int n, int max_entries) {
   return (size_t)(((n - 1) >> coarse_shift(n, max_entries)) + 1) * sizeof(int);
 }
 
@@ -1310,8 +1398,12 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
   int* Os = a.Os_out ? a.Os_out : s.Os;
   unsigned* c = s.counters;
   if (!a.max_known && a.kind != BPF_RESAMPLER_METROPOLIS) {
-    int rc = launch_lw_reduce(a.lw, n, s, st);
-    if (rc) return rc;
+    // up to four blocks per SM, at least 2048 log-weights each
+    int blocks = (n + 2047) / 2048;
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    if (blocks > s.max_partials) blocks = s.max_partials;
+    k_lw_max<<<blocks, kBlock, 0, st>>>(a.lw, n, s.partials, s.stats, s.counters);
+    BPF_TRY(cudaGetLastError());
   }
   switch (a.kind) {
     case BPF_RESAMPLER_SYSTEMATIC: {
@@ -1320,14 +1412,13 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
         if (rc != BPF_E_INVALID) return rc;  // BPF_E_INVALID: cooperative launch unavailable, use the passes
       }
       k_weight_tile_sums<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_sum, s.tile_prefix, 0, nullptr,
-                                               a.seed, a.step, nullptr, nullptr, c + 0, a.gate);
+                                               a.seed, a.step, nullptr, nullptr, nullptr, nullptr, c + 0, a.gate);
       k_systematic_offspring<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_prefix, a.uniforms, a.seed,
                                                    a.step, Os, s.zcount, s.zprefix, c + 1, a.gate);
       if (a.permute) {
-        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.etile, coarse_shift(n), s.slot,
-                                                  s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, fill_smem(n), st>>>(a.as, s.E, s.etile, coarse_shift(n),
-                                                                             s.slot, s.zprefix, n, T, s.stats, a.gate);
+        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
+        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
+                                                                 a.gate);
       } else {
         k_ancestors_from_Os<<<grid_stride_blocks(n), kBlock, 0, st>>>(Os, n, a.as, s.stats, a.gate);
       }
@@ -1335,19 +1426,18 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
     }
     case BPF_RESAMPLER_MULTINOMIAL: {
       k_weight_tile_sums<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_sum, s.tile_prefix, 1, a.uniforms,
-                                               a.seed, a.step, s.vtile_sum, s.vtile_prefix, c + 0, a.gate);
-      k_multinomial_prepare<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_prefix, s.vtile_prefix,
-                                                  a.uniforms, a.seed, a.step, s.Ws, s.lu, a.gate);
+                                               a.seed, a.step, s.vtile_sum, s.vtile_prefix,
+                                               reinterpret_cast<unsigned long long*>(s.Ws), s.lu, c + 0, a.gate);
+      k_multinomial_prepare<<<T, kBlock, 0, st>>>(n, s.stats, s.tile_prefix, s.vtile_prefix, s.Ws, s.lu, a.gate);
       k_multinomial_search<<<grid_stride_blocks(n), kBlock, 0, st>>>(s.Ws, s.lu, n, a.as, s.stats, a.gate);
       if (a.permute || a.Os_out) {
         k_offspring_from<<<T, kBlock, 0, st>>>(a.as, n, 1, s.stats, nullptr, Os, s.zcount, s.zprefix, c + 1,
                                                a.gate);
       }
       if (a.permute) {
-        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.etile, coarse_shift(n), s.slot,
-                                                  s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, fill_smem(n), st>>>(a.as, s.E, s.etile, coarse_shift(n),
-                                                                             s.slot, s.zprefix, n, T, s.stats, a.gate);
+        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
+        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
+                                                                 a.gate);
       }
       break;
     }
@@ -1362,10 +1452,9 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
                                                a.gate);
       }
       if (a.permute) {
-        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.etile, coarse_shift(n), s.slot,
-                                                  s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, fill_smem(n), st>>>(a.as, s.E, s.etile, coarse_shift(n),
-                                                                             s.slot, s.zprefix, n, T, s.stats, a.gate);
+        k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
+        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
+                                                                 a.gate);
       }
       break;
     }

@@ -95,6 +95,23 @@ __device__ __forceinline__ int block_exclusive_scan_int_nt(int v, int* total) {
   return r;
 }
 
+// log(ua) < d for the uniform ua of the words (hi, lo) (bpf_u01d).  A
+// single-precision logarithm of the high word decides unless the two are
+// within 1e-4 + 1e-5 |d| (or ua < 2^-16, or d is NaN): hi alone is within
+// 2^-17 of ua relatively, lg2.approx within 2^-22, so the bound holds with
+// more than a factor of ten to spare.  The exact comparison, some 80
+// instructions, is left to one step in thousands.
+__device__ __forceinline__ bool metropolis_accept(uint32_t hi, uint32_t lo, double d) {
+  if (hi >= (1u << 16)) {
+    const float t = __log2f(((float)hi + 0.5f) * 2.3283064365386963e-10f /* 2^-32 */) * 0.6931472f;
+    const float df = (float)d;
+    const float margin = 1e-4f + 1e-5f * fabsf(df);
+    if (t < df - margin) return true;
+    if (t > df + margin) return false;
+  }
+  return log(bpf_u01d(hi, lo)) < d;
+}
+
 // Metropolis ancestor of particle p after B steps, following
 // MetropolisResamplerHost::ancestors
 // (share/src/bi/host/resampler/MetropolisResamplerHost.hpp:290-321); draw k
@@ -106,21 +123,20 @@ __device__ __forceinline__ int metropolis_ancestor(const double* __restrict__ lw
   int p1 = p;
   double lw1 = lw[p];
   for (int k = 0; k < B; ++k) {
-    double ui, ua;
+    double ui;
+    bpf_u32x4 r{};
     if (u) {
-      size_t idx = 2 * ((size_t)p * B + k);
-      ui = u[idx];
-      ua = u[idx + 1];
+      ui = u[2 * ((size_t)p * B + k)];
     } else {
-      bpf_u32x4 r = bpf_draw(seed, (uint32_t)p, (uint32_t)step, (uint32_t)k, BPF_RNG_METROPOLIS);
+      r = bpf_draw(seed, (uint32_t)p, (uint32_t)step, (uint32_t)k, BPF_RNG_METROPOLIS);
       ui = bpf_u01d(r.v[0], r.v[1]);
-      ua = bpf_u01d(r.v[2], r.v[3]);
     }
     int p2 = __double2int_rz(__dmul_rn(ui, nd));
     p2 = p2 < n - 1 ? p2 : n - 1;  // uniformInt(0, n-1); also bounds caller-supplied uniforms
     p2 = p2 > 0 ? p2 : 0;
     double lw2 = __ldg(lw + p2);
-    if (log(ua) < __dsub_rn(lw2, lw1)) {
+    const double d = __dsub_rn(lw2, lw1);
+    if (u ? log(u[2 * ((size_t)p * B + k) + 1]) < d : metropolis_accept(r.v[2], r.v[3], d)) {
       p1 = p2;
       lw1 = lw2;
     }
