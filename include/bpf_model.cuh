@@ -573,14 +573,16 @@ __device__ __forceinline__ void ode_rk43(ParticleVars<B, T>& v, VarAccess<B, T>&
       for (int j = 0; j < N; ++j) r1[j] = old[j];
     }
     if (t < t2) {
-      const T logfac11 = F::mul_(expo, bi::log(e2));
+      const T loge2 = bi::log(e2);
+      const T logfac11 = F::mul_(expo, loge2);
       if (e2 > (T)1) {
         h = F::mul_(h, bi::max(facl, bi::exp(logsafe - logfac11)));
       } else {
         T fac = bi::exp(F::fma_(beta, logfacold, logsafe) - logfac11);
         fac = bi::min(facr, bi::max(facl, fac));
         h = F::mul_(h, fac);
-        logfacold = F::mul_((T)0.5, bi::log(bi::max(e2, (T)1.0e-8)));
+        // 0.5 log(max(e2, 1e-8)): the logarithm at hand, or the bound's
+        logfacold = F::mul_((T)0.5, e2 >= (T)1.0e-8 ? loge2 : bi::log((T)1.0e-8));
       }
     }
     ++nst;

@@ -229,6 +229,7 @@ __device__ __forceinline__ void pz_advance(T& P, T& Z, T alpha, double t1d, doub
   const T t2 = (T)t2d;
   T t = (T)t1d, h = (T)prm.h0;
   T logfacold = Prec<T>::log_((T)1.0e-4);
+  const T logmin = Prec<T>::log_((T)1.0e-8);
   T oP = P, oZ = Z;     // old
   T r1P = P, r1Z = Z;   // r1 (stored state after stage 1, 3, 5)
   int nst = 0;
@@ -279,14 +280,16 @@ __device__ __forceinline__ void pz_advance(T& P, T& Z, T alpha, double t1d, doub
       r1P = oP; r1Z = oZ;
     }
     if (t < t2) {
-      T logfac11 = Prec<T>::mul_(expo, Prec<T>::log_(e2));
+      const T loge2 = Prec<T>::log_(e2);
+      T logfac11 = Prec<T>::mul_(expo, loge2);
       if (e2 > (T)1) {
         h = Prec<T>::mul_(h, fmax(facl, Prec<T>::exp_(logsafe - logfac11)));
       } else {
         T fac = Prec<T>::exp_(Prec<T>::fma_(beta, logfacold, logsafe) - logfac11);
         fac = fmin(facr, fmax(facl, fac));
         h = Prec<T>::mul_(h, fac);
-        logfacold = Prec<T>::mul_((T)0.5, Prec<T>::log_(fmax(e2, (T)1.0e-8)));
+        // 0.5 log(max(e2, 1e-8)): the logarithm at hand, or the bound's
+        logfacold = Prec<T>::mul_((T)0.5, e2 >= (T)1.0e-8 ? loge2 : logmin);
       }
     }
     ++nst;

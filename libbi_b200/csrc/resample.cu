@@ -239,7 +239,7 @@ k_lw_max(const double* __restrict__ lw, int n, LwPartial* partials, StepStats* s
     if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
     __syncthreads();
     m = warp_max((threadIdx.x & 31) < kBlock / 32 ? s_m[threadIdx.x & 31] : -INFINITY);
-    if (pass == 1) break;
+    if (pass == 1 || gridDim.x == 1) break;  // one block's maximum is the result
     if (threadIdx.x == 0) {
       partials[blockIdx.x].mx = m;
       __threadfence();
