@@ -575,37 +575,49 @@ int tune_batch_resample(const BatchFilter* filt, ResamplePlan* p, int ld, cudaSt
     if (cudaGetLastError() != cudaSuccess) rc = BPF_E_CUDA;
   }
   // the candidates take turns, round after round, so that a drift of clocks
-  // or caches during the tuning reaches every one alike; medians decide
+  // or caches during the tuning reaches every one alike; medians decide, among
+  // those that the first round left within kNear of its best.  The first
+  // launch of each thread count, which loads its code, is not timed.
   constexpr int kReps = 3, kMax = 12;
+  constexpr float kNear = 1.25f;
   ResamplePlan c[kMax];
-  float t[kMax][kReps];
+  float t[kMax][kReps], med[kMax];
+  bool in[kMax];
   int nc = 0;
   for (int g = p->group; g <= kGroup; g *= 2)
     for (int thr = 256; thr <= 1024; thr *= 2) {
       c[nc] = *p;
       c[nc].group = g;
-      c[nc++].threads = thr;
+      c[nc].threads = thr;
+      in[nc++] = true;
     }
-  for (int r = -1; !rc && r < kReps; ++r) {  // an untimed round first
+  for (int k = 0; !rc && k < 3; ++k) rc = launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st);
+  for (int r = 0; !rc && r < kReps; ++r) {
     for (int k = 0; !rc && k < nc; ++k) {
-      if (r >= 0 && cudaEventRecord(e0, st) != cudaSuccess) { rc = BPF_E_CUDA; break; }
+      if (!in[k]) continue;
+      if (cudaEventRecord(e0, st) != cudaSuccess) { rc = BPF_E_CUDA; break; }
       rc = launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st);
-      if (!rc && r >= 0 &&
-          (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-           cudaEventElapsedTime(&t[k][r], e0, e1) != cudaSuccess))
+      if (!rc && (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+                  cudaEventElapsedTime(&t[k][r], e0, e1) != cudaSuccess))
         rc = BPF_E_CUDA;
+    }
+    if (r == 0 && !rc) {
+      float least = t[0][0];
+      for (int k = 1; k < nc; ++k) least = std::min(least, t[k][0]);
+      for (int k = 0; k < nc; ++k) in[k] = t[k][0] <= kNear * least;
     }
   }
   if (!rc) {
-    int best = 0;
+    int best = -1;
     for (int k = 0; k < nc; ++k) {
-      std::sort(t[k], t[k] + kReps);
-      if (t[k][kReps / 2] < t[best][kReps / 2]) best = k;
+      if (in[k]) std::sort(t[k], t[k] + kReps);
+      med[k] = t[k][in[k] ? kReps / 2 : 0];
+      if (in[k] && (best < 0 || med[k] < med[best])) best = k;
     }
     *p = c[best];
-    // the thread counts' medians with the kept cluster size
+    // the thread counts' times with the kept cluster size
     if (us)
-      for (int k = 0; k < 3; ++k) us[k] = 1e3 * t[best / 3 * 3 + k][kReps / 2];
+      for (int k = 0; k < 3; ++k) us[k] = 1e3 * med[best / 3 * 3 + k];
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);

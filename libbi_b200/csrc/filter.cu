@@ -410,7 +410,10 @@ static int one_filter_plan(bpf_handle* h, int resampler) {
   int rc = bpf::tune_batch_resample(h->one_filt, &h->one_plan, h->ld, h->stream, nullptr);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(mu);
-  tuned[key] = h->one_plan;
+  bpf::ResamplePlan& kept = tuned[key];  // the shape alone, not this handle's tables
+  kept = h->one_plan;
+  kept.order = nullptr;
+  kept.sorted = nullptr;
   return BPF_OK;
 }
 
