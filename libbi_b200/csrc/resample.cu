@@ -189,11 +189,29 @@ __device__ __forceinline__ int upper_bound_in(const T* __restrict__ A, int lo, i
   return lo;
 }
 
-template <class T>
-__device__ __forceinline__ int block_upper_bound(const T* __restrict__ A, int n, T x, T x_first, T x_last) {
+// K searches per thread side by side, so that their loads are in flight
+// together: answers in [b, b + len], the same len for all.
+template <int K, class T>
+__device__ __forceinline__ void block_upper_bounds(const T* __restrict__ A, int n, const T (&x)[K], T x_first, T x_last,
+                                                   int (&b)[K]) {
   int bound[2];
   block_bounds(A, n, x_first, x_last, bound);
-  return upper_bound_in(A, bound[0], bound[1], x);
+  int len = bound[1] - bound[0];
+#pragma unroll
+  for (int k = 0; k < K; ++k) b[k] = bound[0];
+  while (len > 1) {
+    const int half = len >> 1;
+    T v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = __ldg(A + b[k] + half - 1);
+#pragma unroll
+    for (int k = 0; k < K; ++k) b[k] = v[k] > x[k] ? b[k] : b[k] + half;
+    len -= half;
+  }
+  if (len == 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) b[k] += __ldg(A + b[k]) > x[k] ? 0 : 1;
+  }
 }
 
 __device__ __forceinline__ bool gate_closed(const int* gate, const StepStats* st) {
@@ -264,46 +282,91 @@ k_lw_max(const double* __restrict__ lw, int n, LwPartial* partials, StepStats* s
 // ---------------------------------------------------------------------------
 // weight tile sums (+ spacing tile sums for multinomial)
 // ---------------------------------------------------------------------------
+// Block-wide sums of one u128 per thread of each of NV values (blockDim.x ==
+// kBlock), in thread 0: exact, so any order gives the same.
+template <int NV>
+__device__ __forceinline__ void block_sum_u128(u128 (&v)[NV]) {
+  __shared__ u128 ws[NV][kBlock / 32];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      u128 o;
+      o.lo = __shfl_xor_sync(0xffffffffu, v[j].lo, d);
+      o.hi = __shfl_xor_sync(0xffffffffu, v[j].hi, d);
+      v[j] = u128_add(v[j], o);
+    }
+    if ((threadIdx.x & 31) == 0) ws[j][threadIdx.x >> 5] = v[j];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      for (int w = 1; w < kBlock / 32; ++w) v[j] = u128_add(v[j], ws[j][w]);
+  }
+}
+
+// A tile is kBlock * ITEMS particles, consecutive threads on consecutive
+// ones: only the tile's sums are needed, and loads and stores of a warp are
+// then whole lines.  Bound by instruction issue (about 450 a particle with
+// spacings) and the last block's scans of the tiles; at 10^6 particles 21.7
+// us against 28 with tiles of 512 particles, each summed by two block scans,
+// four chunks of which the last block then scanned one after another.
+template <int ITEMS, bool MULT>
 __global__ void __launch_bounds__(kBlock)
 k_weight_tile_sums(const double* __restrict__ lw, int n, StepStats* st,
                    u128* tile_sum, u128* tile_prefix,
-                   int with_spacings, const double* u, uint64_t seed, int step,
+                   const double* u, uint64_t seed, int step,
                    u128* vtile_sum, u128* vtile_prefix, unsigned long long* qbuf, double* spbuf,
                    unsigned* counter, const int* gate) {
   if (gate_closed(gate, st)) return;
   const double mx = st->mx;
   const int t = blockIdx.x;
-  const int i0 = t * kTile + threadIdx.x * kItems;
-  double v[kItems];
-  load_blocked(lw, i0, n, v);
-  u128 acc = u128_zero(), vacc = u128_zero();
+  const long long i0 = (long long)t * (kBlock * ITEMS) + threadIdx.x;
+  u128 acc[MULT ? 2 : 1];
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    if (i0 + k < n) {
-      double w = nanexp(__dsub_rn(v[k], mx));
-      u128 q; q.lo = weight_to_fixed(w); q.hi = 0;
-      acc = u128_add(acc, q);
-      if (with_spacings) {
-        // kept for k_multinomial_prepare: 16 bytes against an exp, a draw, a
-        // logarithm and a division
-        const double sp = multinomial_spacing(u, i0 + k, n, seed, step);
-        vacc = u128_add(vacc, spacing_to_fixed(sp));
-        qbuf[i0 + k] = q.lo;
-        spbuf[i0 + k] = sp;
+  for (int j = 0; j < (MULT ? 2 : 1); ++j) acc[j] = u128_zero();
+  double nx[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) nx[j] = i0 + j * kBlock < n ? __ldg(lw + i0 + j * kBlock) : 0.0;
+  // two particles at a time, the next two's log-weights in flight: unrolled
+  // further, the code (an exp, a draw, a logarithm and a division each) no
+  // longer fits the instruction cache
+#pragma unroll 1
+  for (int k = 0; k < ITEMS; k += 2) {
+    double v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      v[j] = nx[j];
+      const long long in = i0 + (k + 2 + j) * kBlock;
+      if (k + 2 < ITEMS) nx[j] = in < n ? __ldg(lw + in) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const long long i = i0 + (k + j) * kBlock;
+      if (i < n) {
+        const double w = nanexp(__dsub_rn(v[j], mx));
+        u128 q; q.lo = weight_to_fixed(w); q.hi = 0;
+        acc[0] = u128_add(acc[0], q);
+        if (MULT) {
+          // kept for k_multinomial_prepare: 16 bytes against an exp, a draw,
+          // a logarithm and a division
+          const double sp = multinomial_spacing(u, (int)i, n, seed, step);
+          acc[MULT ? 1 : 0] = u128_add(acc[MULT ? 1 : 0], spacing_to_fixed(sp));
+          qbuf[i] = q.lo;
+          spbuf[i] = sp;
+        }
       }
     }
   }
-  u128 tot;
-  block_exclusive_scan_u128(acc, &tot);
-  if (threadIdx.x == 0) tile_sum[t] = tot;
-  if (with_spacings) {
-    u128 vtot;
-    block_exclusive_scan_u128(vacc, &vtot);
-    if (threadIdx.x == 0) vtile_sum[t] = vtot;
+  block_sum_u128(acc);
+  if (threadIdx.x == 0) {
+    tile_sum[t] = acc[0];
+    if (MULT) vtile_sum[t] = acc[MULT ? 1 : 0];
   }
   if (last_block_arrive(counter)) {
     block_scan_tiles_u128(tile_sum, tile_prefix, gridDim.x);
-    if (with_spacings) block_scan_tiles_u128(vtile_sum, vtile_prefix, gridDim.x);
+    if (MULT) block_scan_tiles_u128(vtile_sum, vtile_prefix, gridDim.x);
     __syncthreads();
     if (threadIdx.x == 0) {
       *counter = 0;
@@ -1181,29 +1244,37 @@ k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* 
 // Childless slot of rank r receives the ancestor a with E_a <= r < E_{a+1}.
 // One thread per rank, so the work is balanced however the copies are
 // distributed.
+template <int K>
 __global__ void __launch_bounds__(kBlock)
 k_permute_fill(int* as, const int* __restrict__ E, const int* __restrict__ slot, const int* zprefix, int n, int T,
                const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
   const int R = zprefix[T];
-  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < R; b0 += (long long)gridDim.x * kBlock) {
-    const int base = (int)b0;
-    const int r = (int)min(b0 + threadIdx.x, (long long)R - 1);
-    const int a = block_upper_bound(E, n, r, base, (int)min(b0 + kBlock, (long long)R) - 1) - 1;
-    as[__ldg(slot + r)] = a;
+  constexpr int kSpan = kBlock * K;
+  for (long long b0 = (long long)blockIdx.x * kSpan; b0 < R; b0 += (long long)gridDim.x * kSpan) {
+    int r[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) r[k] = (int)min(b0 + k * kBlock + threadIdx.x, (long long)R - 1);
+    block_upper_bounds(E, n, r, (int)b0, (int)min(b0 + kSpan, (long long)R) - 1, b);
+#pragma unroll
+    for (int k = 0; k < K; ++k) as[__ldg(slot + r[k])] = b[k] - 1;
   }
 }
 
 // Unpermuted: as_j = i for Os_{i-1} <= j < Os_i, i.e. upper_bound(Os, j)
 // (ResamplerHost::cumulativeOffspringToAncestors, ResamplerHost.hpp:110-131).
+template <int K>
 __global__ void __launch_bounds__(kBlock)
 k_ancestors_from_Os(const int* __restrict__ Os, int n, int* as, const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
-  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < n; b0 += (long long)gridDim.x * kBlock) {
-    const int base = (int)b0;
-    const int j = (int)min(b0 + threadIdx.x, (long long)n - 1);
-    const int r = block_upper_bound(Os, n, j, base, (int)min(b0 + kBlock, (long long)n) - 1);
-    as[j] = r < n ? r : n - 1;  // Os[n-1] == n for valid offsets; bounds any other
+  constexpr int kSpan = kBlock * K;
+  for (long long b0 = (long long)blockIdx.x * kSpan; b0 < n; b0 += (long long)gridDim.x * kSpan) {
+    int j[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) j[k] = (int)min(b0 + k * kBlock + threadIdx.x, (long long)n - 1);
+    block_upper_bounds(Os, n, j, (int)b0, (int)min(b0 + kSpan, (long long)n) - 1, b);
+#pragma unroll
+    for (int k = 0; k < K; ++k) as[j[k]] = b[k] < n ? b[k] : n - 1;  // Os[n-1] == n for valid offsets; bounds any other
   }
 }
 
@@ -1214,55 +1285,92 @@ k_ancestors_from_Os(const int* __restrict__ Os, int n, int* as, const StepStats*
 // lu_s = log(W) + lMax_s, lMax_s = sum_{i > s} log(u)/i.
 // ---------------------------------------------------------------------------
 // Ws: the fixed-point weights in, the logarithms of the cumulative weights
-// out; lu: the spacings in, the log uniforms out (each thread's own entries).
+// out; lu: the spacings in, the log uniforms out (each thread's own entries,
+// which the buffers' alignment allows in 16-byte pairs).
+template <int ITEMS>
 __global__ void __launch_bounds__(kBlock)
 k_multinomial_prepare(int n, const StepStats* st, const u128* tile_prefix, const u128* vtile_prefix, double* Ws,
                       double* lu, const int* gate) {
+  static_assert(ITEMS % 2 == 0, "entries in pairs");
   if (gate_closed(gate, st)) return;
   const int t = blockIdx.x;
   const int T = gridDim.x;
-  const int i0 = t * kTile + threadIdx.x * kItems;
+  const long long i0 = (long long)t * (kBlock * ITEMS) + threadIdx.x * ITEMS;
   const double lW = log(u128_to_weight(tile_prefix[T]));
   const u128 Vtot = vtile_prefix[T];
-  unsigned long long q[kItems];
-  u128 vv[kItems];
+  unsigned long long q[ITEMS];
+  double sp[ITEMS];
   u128 loc = u128_zero(), vloc = u128_zero();
+  if (i0 + ITEMS <= n) {
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    const bool in = i0 + k < n;
-    q[k] = in ? reinterpret_cast<const unsigned long long*>(Ws)[i0 + k] : 0ull;
-    vv[k] = in ? spacing_to_fixed(lu[i0 + k]) : u128_zero();
+    for (int k = 0; k < ITEMS; k += 2) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(Ws + i0 + k);
+      const double2 b = *reinterpret_cast<const double2*>(lu + i0 + k);
+      q[k] = a.x; q[k + 1] = a.y;
+      sp[k] = b.x; sp[k + 1] = b.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      q[k] = i0 + k < n ? reinterpret_cast<const unsigned long long*>(Ws)[i0 + k] : 0ull;
+      sp[k] = i0 + k < n ? lu[i0 + k] : 0.0;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
     u128 qq; qq.lo = q[k]; qq.hi = 0;
     loc = u128_add(loc, qq);
-    vloc = u128_add(vloc, vv[k]);
+    vloc = u128_add(vloc, spacing_to_fixed(sp[k]));
   }
   u128 tot, vtot;
   u128 Q = u128_add(tile_prefix[t], block_exclusive_scan_u128(loc, &tot));
   u128 V = u128_add(vtile_prefix[t], block_exclusive_scan_u128(vloc, &vtot));
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    u128 qq; qq.lo = q[k]; qq.hi = 0;
-    Q = u128_add(Q, qq);
-    if (i0 + k < n) {
-      Ws[i0 + k] = log(u128_to_weight(Q));
+  for (int k = 0; k < ITEMS; k += 2) {
+    double2 w, l;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      u128 qq; qq.lo = q[k + j]; qq.hi = 0;
+      Q = u128_add(Q, qq);
+      const double lq = log(u128_to_weight(Q));
       // suffix sum over slots >= s of the spacings, then lu = lW + lMax
-      double lmax = -fixed_to_spacing(u128_sub(Vtot, V));
-      lu[i0 + k] = __dadd_rn(lW, lmax);
+      const double ls = __dadd_rn(lW, -fixed_to_spacing(u128_sub(Vtot, V)));
+      V = u128_add(V, spacing_to_fixed(sp[k + j]));
+      (j ? w.y : w.x) = lq;
+      (j ? l.y : l.x) = ls;
     }
-    V = u128_add(V, vv[k]);
+    if (i0 + k + 2 <= n) {
+      *reinterpret_cast<double2*>(Ws + i0 + k) = w;
+      *reinterpret_cast<double2*>(lu + i0 + k) = l;
+    } else if (i0 + k < n) {
+      Ws[i0 + k] = w.x;
+      lu[i0 + k] = l.x;
+    }
   }
 }
 
+// Bound by the latency of the searches' loads from L2: one bracketing and one
+// round of ten dependent loads per 1024 slots, all blocks of 10^6 particles
+// resident at once: 13.2 us against 21.9 with one slot per thread.
+template <int K>
 __global__ void __launch_bounds__(kBlock)
 k_multinomial_search(const double* __restrict__ lWs, const double* __restrict__ lu, int n, int* as,
                      const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
-  for (long long b0 = (long long)blockIdx.x * kBlock; b0 < n; b0 += (long long)gridDim.x * kBlock) {
+  constexpr int kSpan = kBlock * K;
+  for (long long b0 = (long long)blockIdx.x * kSpan; b0 < n; b0 += (long long)gridDim.x * kSpan) {
     const int base = (int)b0;
-    const int s = (int)min(b0 + threadIdx.x, (long long)n - 1);
-    const int r = block_upper_bound(lWs, n, lu[s], lu[base], lu[(int)min(b0 + kBlock, (long long)n) - 1]);
+    int s[K], b[K];
+    double x[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      s[k] = (int)min(b0 + k * kBlock + threadIdx.x, (long long)n - 1);
+      x[k] = __ldg(lu + s[k]);
+    }
+    block_upper_bounds(lWs, n, x, __ldg(lu + base), __ldg(lu + (int)min(b0 + kSpan, (long long)n) - 1), b);
     // the reference's loop can leave j = n when lu rounds up to log(W); clamp
-    as[s] = r < n ? r : n - 1;
+#pragma unroll
+    for (int k = 0; k < K; ++k) as[s[k]] = b[k] < n ? b[k] : n - 1;
   }
 }
 
@@ -1391,6 +1499,37 @@ static inline int grid_stride_blocks(int n) {
   return b < 148 * 8 ? (b > 0 ? b : 1) : 148 * 8;
 }
 
+// The kernels that search for each slot, with K searches per thread: one
+// while all blocks are resident at once (148 SMs x 8), kWide beyond, so that
+// a block's bracketing serves more slots and its searches overlap.
+constexpr int kWide = 4;
+template <class... KArgs, class... Args>
+static void launch_searched(void (*one)(KArgs...), void (*wide)(KArgs...), int n, cudaStream_t st, Args... args) {
+  const int blocks = (n + kBlock - 1) / kBlock, resident = 148 * 8;
+  if (blocks <= resident)
+    one<<<blocks, kBlock, 0, st>>>(args...);
+  else
+    wide<<<std::min((blocks + kWide - 1) / kWide, resident), kBlock, 0, st>>>(args...);
+}
+
+// The multinomial resampler's cumulative weights and log uniforms, in tiles
+// of kBlock * ITEMS particles.  More particles per thread make fewer block
+// sums and scans and fewer tiles for the last block to scan alone, fewer make
+// more blocks.  A whole sorted resampling on B200 with 2 / 4 / 8 per thread:
+// 56 / 57 / 64 us at 2^17 particles, 67 / 62 / 68 at 2^18, 72 / 70 / 67 at
+// 2^19, 94 / 93 / 93 at 10^6, 245 / 217 / 207 at 2^22.
+constexpr int kMultinomial4From = 1 << 18, kMultinomial8From = 1 << 19;
+template <int ITEMS>
+static void launch_multinomial_draws(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) {
+  const int tiles = (a.n + kBlock * ITEMS - 1) / (kBlock * ITEMS);
+  k_weight_tile_sums<ITEMS, true><<<tiles, kBlock, 0, st>>>(a.lw, a.n, s.stats, s.tile_sum, s.tile_prefix, a.uniforms,
+                                                            a.seed, a.step, s.vtile_sum, s.vtile_prefix,
+                                                            reinterpret_cast<unsigned long long*>(s.Ws), s.lu,
+                                                            s.counters, a.gate);
+  k_multinomial_prepare<ITEMS><<<tiles, kBlock, 0, st>>>(a.n, s.stats, s.tile_prefix, s.vtile_prefix, s.Ws, s.lu,
+                                                         a.gate);
+}
+
 int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) {
   if (a.n <= 0 || a.n > s.max_n || a.as == nullptr) return BPF_E_INVALID;
   const int n = a.n;
@@ -1411,33 +1550,34 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
         int rc = launch_systematic_coop(a, s, a.Os_out, st);
         if (rc != BPF_E_INVALID) return rc;  // BPF_E_INVALID: cooperative launch unavailable, use the passes
       }
-      k_weight_tile_sums<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_sum, s.tile_prefix, 0, nullptr,
-                                               a.seed, a.step, nullptr, nullptr, nullptr, nullptr, c + 0, a.gate);
+      k_weight_tile_sums<kItems, false><<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_sum, s.tile_prefix, nullptr,
+                                                              a.seed, a.step, nullptr, nullptr, nullptr, nullptr, c + 0,
+                                                              a.gate);
       k_systematic_offspring<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_prefix, a.uniforms, a.seed,
                                                    a.step, Os, s.zcount, s.zprefix, c + 1, a.gate);
       if (a.permute) {
         k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
-                                                                 a.gate);
+        launch_searched(k_permute_fill<1>, k_permute_fill<kWide>, n, st, a.as, s.E, s.slot, s.zprefix, n, T,
+                        s.stats, a.gate);
       } else {
-        k_ancestors_from_Os<<<grid_stride_blocks(n), kBlock, 0, st>>>(Os, n, a.as, s.stats, a.gate);
+        launch_searched(k_ancestors_from_Os<1>, k_ancestors_from_Os<kWide>, n, st, (const int*)Os, n, a.as, s.stats, a.gate);
       }
       break;
     }
     case BPF_RESAMPLER_MULTINOMIAL: {
-      k_weight_tile_sums<<<T, kBlock, 0, st>>>(a.lw, n, s.stats, s.tile_sum, s.tile_prefix, 1, a.uniforms,
-                                               a.seed, a.step, s.vtile_sum, s.vtile_prefix,
-                                               reinterpret_cast<unsigned long long*>(s.Ws), s.lu, c + 0, a.gate);
-      k_multinomial_prepare<<<T, kBlock, 0, st>>>(n, s.stats, s.tile_prefix, s.vtile_prefix, s.Ws, s.lu, a.gate);
-      k_multinomial_search<<<grid_stride_blocks(n), kBlock, 0, st>>>(s.Ws, s.lu, n, a.as, s.stats, a.gate);
+      if (n >= kMultinomial8From) launch_multinomial_draws<8>(a, s, st);
+      else if (n >= kMultinomial4From) launch_multinomial_draws<4>(a, s, st);
+      else launch_multinomial_draws<2>(a, s, st);
+      launch_searched(k_multinomial_search<1>, k_multinomial_search<kWide>, n, st, (const double*)s.Ws, (const double*)s.lu, n, a.as,
+                      s.stats, a.gate);
       if (a.permute || a.Os_out) {
         k_offspring_from<<<T, kBlock, 0, st>>>(a.as, n, 1, s.stats, nullptr, Os, s.zcount, s.zprefix, c + 1,
                                                a.gate);
       }
       if (a.permute) {
         k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
-                                                                 a.gate);
+        launch_searched(k_permute_fill<1>, k_permute_fill<kWide>, n, st, a.as, s.E, s.slot, s.zprefix, n, T,
+                        s.stats, a.gate);
       }
       break;
     }
@@ -1453,8 +1593,8 @@ int launch_resample(const ResampleArgs& a, ResampleScratch& s, cudaStream_t st) 
       }
       if (a.permute) {
         k_permute_survivors<<<T, kBlock, 0, st>>>(Os, n, s.zprefix, a.as, s.E, s.slot, s.stats, a.gate);
-        k_permute_fill<<<grid_stride_blocks(n), kBlock, 0, st>>>(a.as, s.E, s.slot, s.zprefix, n, T, s.stats,
-                                                                 a.gate);
+        launch_searched(k_permute_fill<1>, k_permute_fill<kWide>, n, st, a.as, s.E, s.slot, s.zprefix, n, T,
+                        s.stats, a.gate);
       }
       break;
     }
