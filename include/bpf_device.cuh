@@ -240,11 +240,13 @@ __device__ __forceinline__ void record_step(StepStats* st, int resampled, bool o
 // the end of every transition block: this block's (max, sum e, sum e^2) to
 // partials[pidx]; the last of the np blocks that share `counter` combines
 // partials[pbase .. pbase + np) and writes the step statistics.  Returns true
-// in the block that finalised.
+// in the block that finalised.  nt: the threads that fold the partials (the
+// first nt of the block; the rest take part empty), so that the order does
+// not depend on a block's size; blockDim.x unless given.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ bool transition_reduce_tail(LwPartial part, LwPartial* partials, int pidx, int pbase,
                                                        int np, unsigned* counter, int n, StepStats* st, bool ok,
-                                                       int resampled, bool observed) {
+                                                       int resampled, bool observed, int nt = 0) {
   // the block's own combination and the last block's share one copy of the
   // code, so that the second finds it in the instruction cache
   __shared__ bool am_last;
@@ -261,7 +263,10 @@ __device__ __forceinline__ bool transition_reduce_tail(LwPartial part, LwPartial
     if (!am_last) return false;
     __threadfence();
     if (!ok) break;
-    part = fold_partials(partials + pbase, np, threadIdx.x, blockDim.x);
+    if (nt == 0)
+      part = fold_partials(partials + pbase, np, threadIdx.x, blockDim.x);
+    else
+      part = threadIdx.x < nt ? fold_partials(partials + pbase, np, threadIdx.x, nt) : lw_empty();
   }
   if (threadIdx.x == 0) {
     if (ok) {

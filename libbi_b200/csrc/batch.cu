@@ -129,6 +129,46 @@ k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld
     batch_record(st, hist, nf, f, k);
 }
 
+// The same with two threads per particle (l96_pair_step), as the single
+// filters' k_l96_transition_pair.
+template <class T, int D, int MB>
+__global__ void __launch_bounds__(2 * kL96Block, MB)
+k_batch_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
+                            double* __restrict__ lw, const T* __restrict__ y, double t1d, double t2d, int step,
+                            const BatchFilter* __restrict__ filt, const L96Params* __restrict__ prms,
+                            const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
+                            double* hist, int nf, int k) {
+  __shared__ T sz[D / 2][2 * kL96Block];
+  const int f = __ldg(blk2f + blockIdx.x);
+  const BatchFilter fd = filt[f];
+  const int p = (blockIdx.x - fd.block0) * kL96Block + (threadIdx.x >> 1);
+  l96_pair_draw<T, D>(sz, fd.seed, (uint32_t)p, step);
+  pdl_wait();  // the resampler's ancestors and statistics
+  StepStats* st = stats + f;
+  const int resampled = st->resample;
+  const bool ok = __syncthreads_and(st->status == BPF_OK) != 0;
+  const T* yf = y ? y + (size_t)f * D : nullptr;
+  LwPartial part = lw_empty();
+  if (ok) {
+    const bool live = p < fd.n;
+    const int col = fd.off + p;
+    const int src = live ? (resampled ? min(max(as[col], 0), fd.n - 1) : p) : 0;
+    l96_pair_step<T, D>(sz, x_in + fd.off, src, x_out, col, ld, live, yf, ~0ull, t1d, t2d, prms[f]);
+    if (resampled && live && (threadIdx.x & 1) == 0) as[col] = src;
+    __syncthreads();
+    const int q = (blockIdx.x - fd.block0) * kL96Block + threadIdx.x;
+    if (threadIdx.x < kL96Block && q < fd.n) {
+      const double l = l96_pair_terms<T, D>(sz, resampled ? st->ll : lw[fd.off + q], y != nullptr, ~0ull);
+      lw[fd.off + q] = l;
+      lw_push(part, l);
+    }
+  }
+  pdl_trigger();
+  if (transition_reduce_tail(part, partials, blockIdx.x, fd.block0, fd.nblocks, counters + f, fd.n, st, ok,
+                             resampled, y != nullptr, kL96Block))
+    batch_record(st, hist, nf, f, k);
+}
+
 template <class T>
 __global__ void __launch_bounds__(kPZBlock)
 k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
@@ -185,12 +225,40 @@ int launch_batch_init(const ModelArgs& m, void* x, int ld, double* lw, const Bat
   return BPF_OK;
 }
 
-#define BATCH_L96_CASE(TT, DD)                                                                              \
-  case DD:                                                                                                  \
-    BPF_TRY(launch_pdl(k_batch_l96_transition<TT, DD>, dim3(blocks), dim3(kL96Block), 0, st, (const TT*)x_in, \
-                       (TT*)x_out, ld, as, lw, (const TT*)y, t1, t2, step, filt, (const L96Params*)prms,     \
-                       blk2f, stats, partials, counters, hist, nf, k));                                       \
-    break;
+#define BATCH_L96_LAUNCH(KERNEL, THREADS)                                                                      \
+  BPF_TRY(launch_pdl(KERNEL, dim3(blocks), dim3(THREADS), 0, st, (const T*)x_in, (T*)x_out, ld, as, lw,        \
+                     (const T*)y, t1, t2, step, filt, (const L96Params*)prms, blk2f, stats, partials, counters, \
+                     hist, nf, k))
+
+template <class T, int D>
+static int batch_l96_transition(const void* x_in, void* x_out, int ld, int* as, double* lw, const void* y, double t1,
+                                double t2, int step, const BatchFilter* filt, const void* prms, const int* blk2f,
+                                int blocks, StepStats* stats, LwPartial* partials, unsigned* counters, double* hist,
+                                int nf, int k, cudaStream_t st) {
+  if constexpr (D % 8 == 0) {
+    const int mb = l96_pair_blocks(sizeof(T), blocks);
+    if (mb == 2) {
+      BATCH_L96_LAUNCH((k_batch_l96_transition_pair<T, D, 2>), 2 * kL96Block);
+      return BPF_OK;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (mb == 3) {
+        BATCH_L96_LAUNCH((k_batch_l96_transition_pair<T, D, 3>), 2 * kL96Block);
+        return BPF_OK;
+      }
+    }
+  }
+  if constexpr (D % 8 != 0 || sizeof(T) == 4) {
+    BATCH_L96_LAUNCH((k_batch_l96_transition<T, D>), kL96Block);
+    return BPF_OK;
+  }
+  return BPF_E_INVALID;
+}
+
+#define BATCH_L96_CASE(TT, DD)                                                                                  \
+  case DD:                                                                                                      \
+    return batch_l96_transition<TT, DD>(x_in, x_out, ld, as, lw, y, t1, t2, step, filt, prms, blk2f, blocks,    \
+                                        stats, partials, counters, hist, nf, k, st);
 
 int launch_batch_transition(const ModelArgs& m, const void* x_in, void* x_out, int ld, int* as, double* lw,
                             const void* y, double t1, double t2, int step, const BatchFilter* filt,

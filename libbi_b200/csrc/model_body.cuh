@@ -128,6 +128,51 @@ __device__ __forceinline__ void l96_rk4(T (&x0)[D], double t1d, double t2d, T F,
   }
 }
 
+// The same on half of the ring's 2 H components per thread, the other half in
+// the lane whose number differs in bit 0 (every lane of the warp takes part):
+// on both sides of a half lie the other's ends.
+template <class T, int H>
+__device__ __forceinline__ void l96_dfdt_half(const T (&x)[H], T (&k)[H], T F) {
+  const T l2 = __shfl_xor_sync(0xffffffffu, x[H - 2], 1), l1 = __shfl_xor_sync(0xffffffffu, x[H - 1], 1),
+          r = __shfl_xor_sync(0xffffffffu, x[0], 1);
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const T xp = i + 1 < H ? x[(i + 1) % H] : r;
+    const T xm = i >= 1 ? x[(i + H - 1) % H] : l1;
+    const T xmm = i >= 2 ? x[(i + H - 2) % H] : i == 1 ? l1 : l2;
+    T d = xp - xmm;
+    k[i] = Prec<T>::fma_(d, xm, -x[i]) + F;
+  }
+}
+
+template <class T, int H>
+__device__ __forceinline__ void l96_rk4_half(T (&x0)[H], double t1d, double t2d, T F, T h0) {
+  const T b1 = (T)(1.0 / 6.0), b2 = (T)(1.0 / 3.0), b3 = (T)(1.0 / 3.0), b4 = (T)(1.0 / 6.0);
+  const T t2 = (T)t2d;
+  T t = (T)t1d, h = h0;
+  while (t < t2) {
+    if (Prec<T>::fma_((T)1.01, h, t) - t2 > (T)0) {
+      h = t2 - t;
+      if (h <= (T)0) { t = t2; break; }
+    }
+    const T hh = (T)0.5 * h;
+    T xs[H], k[H], acc[H];
+    l96_dfdt_half<T, H>(x0, k, F);
+#pragma unroll
+    for (int i = 0; i < H; ++i) { acc[i] = b1 * k[i]; xs[i] = Prec<T>::fma_(hh, k[i], x0[i]); }
+    l96_dfdt_half<T, H>(xs, k, F);
+#pragma unroll
+    for (int i = 0; i < H; ++i) { acc[i] = Prec<T>::fma_(b2, k[i], acc[i]); xs[i] = Prec<T>::fma_(hh, k[i], x0[i]); }
+    l96_dfdt_half<T, H>(xs, k, F);
+#pragma unroll
+    for (int i = 0; i < H; ++i) { acc[i] = Prec<T>::fma_(b3, k[i], acc[i]); xs[i] = Prec<T>::fma_(h, k[i], x0[i]); }
+    l96_dfdt_half<T, H>(xs, k, F);
+#pragma unroll
+    for (int i = 0; i < H; ++i) { acc[i] = Prec<T>::fma_(b4, k[i], acc[i]); x0[i] = Prec<T>::fma_(h, acc[i], x0[i]); }
+    t += h;
+  }
+}
+
 // eta[i] ~ gaussian(0, sigma_eta); x[i] <- x[i] + eta[i]; then
 // lp += -0.5*((y - x)/sigma)^2 - BI_HALF_LOG_TWO_PI - log(sigma), four
 // components per Philox block, in component order.  The integrated state is
@@ -177,6 +222,95 @@ __device__ __forceinline__ double l96_noise_obs(const T (&sx)[D][kL96Block], T* 
   if ((mask & all) == all)
     return l96_noise_obs_impl<T, D, false>(sx, x_out, ld, p_out, y, seed, prng, step, prm, l, mask);
   return l96_noise_obs_impl<T, D, true>(sx, x_out, ld, p_out, y, seed, prng, step, prm, l, mask);
+}
+
+// ---------------------------------------------------------------------------
+// The Lorenz '96 step with two threads per particle: adjacent lanes, thread
+// 2 r + half of a block of 2 kL96Block holding components [half D/2,
+// (half + 1) D/2) of the block's particle r.  While the blocks of a launch
+// are all resident at once, its time is the latency of a thread's
+// instructions (at N = 20011 in FP64 one warp per scheduler issued every
+// fourth cycle, the FP64 pipe 28 % busy), which this halves; the draws, which
+// need nothing of the kernel before, come before the wait for it.  Same
+// arithmetic, and one thread per particle adds its terms and enters the
+// reduction, so the same bits.
+// ---------------------------------------------------------------------------
+// Blocks of the two-thread form on an SM for a launch of `blocks` blocks, or 0
+// for one thread per particle.  Microseconds per filter step on B200 (d = 40,
+// resampler included), one thread / two threads: FP32 25.3 / 21.2 at N = 4096,
+// 31.7 / 27.1 at 18944, 37.6 / 30.3 at 37888 (two blocks on every SM; 36.6
+// compiled for three), 44.3 / 38.0 at 56832 (three), 44.4 / 46.7 at 65536 (a
+// second wave); FP64 33.8 / 24.8 at 4096, 40.8 / 33.9 at 20011, 69.1 / 60.8 at
+// 65536, 699 / 643 at 10^6: there one thread's 255 registers leave an SM half
+// the warps at any size.
+inline int l96_pair_blocks(int esz, int blocks) {
+  if (esz == 8) return 2;
+  return blocks <= 2 * 148 ? 2 : blocks <= 3 * 148 ? 3 : 0;
+}
+
+// the thread's draws, by component
+template <class T, int D>
+__device__ __forceinline__ void l96_pair_draw(T (&sz)[D / 2][2 * kL96Block], uint64_t seed, uint32_t prng, int step) {
+  static_assert(D % 8 == 0, "a Philox block's four components belong to one thread");
+  const int tid = threadIdx.x, half = tid & 1;
+#pragma unroll 1
+  for (int b = 0; b < D / 8; ++b) {
+    const bpf_u32x4 r = bpf_draw(seed, prng, (uint32_t)step, (uint32_t)(half * (D / 8) + b), BPF_RNG_NOISE);
+    T z[4];
+    box_muller4(r, z);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sz[4 * b + j][tid] = z[j];
+  }
+}
+
+// The thread's half of the particle's state from column src of x_in, advanced,
+// to column p of x_out; the observation terms take the draws' place.  Every
+// thread of the block calls it (the halves meet in shuffles).
+template <class T, int D>
+__device__ __forceinline__ void l96_pair_step(T (&sz)[D / 2][2 * kL96Block], const T* __restrict__ x_in, int src,
+                                              T* __restrict__ x_out, int p, int ld, bool live,
+                                              const T* __restrict__ y, uint64_t mask, double t1d, double t2d,
+                                              const L96Params& prm) {
+  constexpr int H = D / 2;
+  constexpr uint64_t all = (1ull << D) - 1ull;
+  const bool full = (mask & all) == all;
+  const int tid = threadIdx.x, c0 = (tid & 1) * H;
+  T x0[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i) x0[i] = live ? __ldg(x_in + (size_t)(c0 + i) * ld + src) : (T)0;
+  l96_rk4_half<T, H>(x0, t1d, t2d, (T)prm.F, (T)prm.h);
+  if (!live) return;
+  const T se = (T)prm.sigma_eta;
+  const T sy = (T)prm.sigma_y, isy = (T)prm.inv_sigma_y;
+  const T c2 = (T)prm.c_half_log_2pi, ls = (T)prm.log_sigma_y;
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const T xi = Prec<T>::add_(x0[i], Prec<T>::mul_(se, sz[i][tid]));
+    x_out[(size_t)(c0 + i) * ld + p] = xi;
+    if (y && (full || ((mask >> (c0 + i)) & 1ull))) {
+      T dz = __ldg(y + c0 + i) - xi;
+      dz = isy != (T)0 ? dz * isy : dz / sy;
+      sz[i][tid] = Prec<T>::fma_((T)-0.5, dz * dz, -c2) - ls;
+    }
+  }
+}
+
+// l plus the observation terms of the block's particle threadIdx.x, in
+// component order
+template <class T, int D>
+__device__ __forceinline__ double l96_pair_terms(const T (&sz)[D / 2][2 * kL96Block], double l, bool observed,
+                                                 uint64_t mask) {
+  constexpr int H = D / 2;
+  constexpr uint64_t all = (1ull << D) - 1ull;
+  const bool full = (mask & all) == all;
+  if (!observed) return l;
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+#pragma unroll
+    for (int i = 0; i < H; ++i)
+      if (full || ((mask >> (s * H + i)) & 1ull)) l += (double)sz[i][2 * threadIdx.x + s];
+  }
+  return l;
 }
 
 // ---------------------------------------------------------------------------

@@ -50,21 +50,54 @@ k_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int 
   transition_reduce_tail(part, partials, blockIdx.x, 0, gridDim.x, counter, n, st, ok, resampled, y != nullptr);
 }
 
+// The same with two threads per particle (l96_pair_step); MB: blocks resident
+// on an SM.
+template <class T, int D, int MB>
+__global__ void __launch_bounds__(2 * kL96Block, MB)
+k_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n,
+                      int* __restrict__ as, double* __restrict__ lw, const T* __restrict__ y,
+                      double t1d, double t2d, uint64_t seed, int step, L96Params prm,
+                      StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask) {
+  __shared__ T sz[D / 2][2 * kL96Block];
+  const int p = blockIdx.x * kL96Block + (threadIdx.x >> 1);
+  l96_pair_draw<T, D>(sz, seed, (uint32_t)p, step);
+  pdl_wait();  // the resampler's ancestors and statistics
+  const int resampled = st->resample;
+  const bool ok = __syncthreads_and(st->status == BPF_OK) != 0;
+  LwPartial part = lw_empty();
+  if (ok) {
+    const int src = p < n ? (resampled ? as[p] : p) : 0;
+    l96_pair_step<T, D>(sz, x_in, src, x_out, p, ld, p < n, y, mask, t1d, t2d, prm);
+    if (resampled && p < n && (threadIdx.x & 1) == 0) as[p] = src;
+    __syncthreads();
+    const int q = blockIdx.x * kL96Block + threadIdx.x;
+    if (threadIdx.x < kL96Block && q < n) {
+      const double l = l96_pair_terms<T, D>(sz, resampled ? st->ll : lw[q], y != nullptr, mask);
+      lw[q] = l;
+      lw_push(part, l);
+    }
+  }
+  pdl_trigger();
+  transition_reduce_tail(part, partials, blockIdx.x, 0, gridDim.x, counter, n, st, ok, resampled, y != nullptr,
+                         kL96Block);
+}
+
 template <class T>
 __global__ void __launch_bounds__(kPZBlock)
 k_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n,
                 int* __restrict__ as, double* __restrict__ lw, const T* __restrict__ y,
                 double t1d, double t2d, uint64_t seed, int step, PZParams prm,
                 StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask) {
-  pdl_wait();  // the resampler's ancestors and statistics
+  // the draw needs nothing of the kernel before
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const T alpha = pz_alpha<T>(seed, (uint32_t)p, step, prm);
+  pdl_wait();  // the resampler's ancestors and statistics
   const int resampled = st->resample;
   const bool ok = st->status == BPF_OK;
   LwPartial part = lw_empty();
   if (p < n && ok) {
     const int src = resampled ? as[p] : p;
     T P = __ldg(x_in + src), Z = __ldg(x_in + (size_t)ld + src);
-    const T alpha = pz_alpha<T>(seed, (uint32_t)p, step, prm);
     pz_advance<T>(P, Z, alpha, t1d, t2d, prm);
     double l = resampled ? st->ll : lw[p];
     if (y && (mask & 1ull)) l += pz_obs_term<T>(P, __ldg(y), prm);
@@ -119,29 +152,49 @@ __global__ void k_stats_init(StepStats* st, int n, double ess_rel) {
 // the transitions are launched as programmatic dependents of the resampler
 // before them (measured on B200 at N = 65536: 49.1 against 50.8 us per
 // filter step), so that their blocks are scheduled while it finishes
-#define L96_CASE(DD)                                                                                   \
-  case DD:                                                                                             \
-    BPF_TRY(launch_pdl(k_l96_transition<T, DD>, dim3(blocks), dim3(kL96Block), 0, st, (const T*)a.x_in,     \
-                       (T*)a.x_out, a.ld, a.n, (int*)a.as, a.lw, (const T*)a.y, a.t1, a.t2, a.seed, a.step,   \
-                       prm, a.stats, a.partials, a.counter, a.obs_mask));                               \
-    break;
+#define L96_LAUNCH(KERNEL, THREADS)                                                                           \
+  BPF_TRY(launch_pdl(KERNEL, dim3(blocks), dim3(THREADS), 0, st, (const T*)a.x_in, (T*)a.x_out, a.ld, a.n,    \
+                     (int*)a.as, a.lw, (const T*)a.y, a.t1, a.t2, a.seed, a.step, prm, a.stats, a.partials,   \
+                     a.counter, a.obs_mask))
+
+template <class T, int D>
+static int l96_transition(const ModelArgs& m, const TransitionArgs& a, int blocks, cudaStream_t st) {
+  const L96Params prm = l96_params<T>(m.theta, m.h);
+  if constexpr (D % 8 == 0) {
+    const int mb = l96_pair_blocks(sizeof(T), blocks);
+    if (mb == 2) {
+      L96_LAUNCH((k_l96_transition_pair<T, D, 2>), 2 * kL96Block);
+      return BPF_OK;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (mb == 3) {
+        L96_LAUNCH((k_l96_transition_pair<T, D, 3>), 2 * kL96Block);
+        return BPF_OK;
+      }
+    }
+  }
+  if constexpr (D % 8 != 0 || sizeof(T) == 4) {
+    L96_LAUNCH((k_l96_transition<T, D>), kL96Block);
+    return BPF_OK;
+  }
+  return BPF_E_INVALID;
+}
 
 template <class T>
 static int transition_t(const ModelArgs& m, const TransitionArgs& a, cudaStream_t st) {
   if (m.kind == BPF_MODEL_L96) {
-    // one particle per thread: 64-thread blocks spread evenly over the SMs
     const int blocks = (a.n + kL96Block - 1) / kL96Block;
     if (blocks > a.max_partials) return BPF_E_INVALID;
-    L96Params prm = l96_params<T>(m.theta, m.h);
+    int rc;
     switch (m.dim) {
-      L96_CASE(4)
-      L96_CASE(8)
-      L96_CASE(16)
-      L96_CASE(32)
-      L96_CASE(40)
-      default:
-        return BPF_E_INVALID;
+      case 4: rc = l96_transition<T, 4>(m, a, blocks, st); break;
+      case 8: rc = l96_transition<T, 8>(m, a, blocks, st); break;
+      case 16: rc = l96_transition<T, 16>(m, a, blocks, st); break;
+      case 32: rc = l96_transition<T, 32>(m, a, blocks, st); break;
+      case 40: rc = l96_transition<T, 40>(m, a, blocks, st); break;
+      default: return BPF_E_INVALID;
     }
+    if (rc) return rc;
   } else if (m.kind == BPF_MODEL_PZ) {
     const int blocks = (a.n + kPZBlock - 1) / kPZBlock;
     if (blocks > a.max_partials) return BPF_E_INVALID;
