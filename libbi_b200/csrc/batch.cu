@@ -7,13 +7,13 @@
 // filters of one model (each with its own particle count, constants, seed and
 // resampler) in shared structure-of-arrays buffers, and one filter step of
 // the whole batch is two launches:
-//   k_batch_resample      one cluster of eight CTAs per filter that resamples
+//   k_batch_resample      one cluster of 1 to 8 CTAs per filter that resamples
 //                         (gated on the filter's own ESS flag): the permuted
 //                         systematic, multinomial or Metropolis ancestors of
 //                         the single-filter path, computed on chip
 //                         (batch_resample.cu)
-//   k_batch_*_transition  one thread per particle over all filters' blocks;
-//                         the last block of each filter finalises that
+//   k_batch_*_transition  one thread per particle (Lorenz-96: or two) over all
+//                         filters' blocks; the last block of each filter finalises that
 //                         filter's ESS, lW, logLikelihood and resample flag
 // Filter f's particles occupy columns [off_f, off_f + n_f) of every state
 // row; its transition blocks never straddle another filter.  Filter f draws

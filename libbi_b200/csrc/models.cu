@@ -1,7 +1,8 @@
 // Model transition + observation kernels of the single bootstrap particle
 // filter (the per-particle bodies are in model_body.cuh).
 //
-// One thread advances one particle through one observation interval, fusing
+// One thread (Lorenz-96: or two, k_l96_transition_pair) advances one particle
+// through one observation interval, fusing
 // the ancestor gather (State::gather -> gather_rows,
 // share/src/bi/state/State.hpp:907-909), the noise draw, the ODE, the
 // deterministic update, the observation log-density and the block partial of

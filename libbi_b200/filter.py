@@ -559,7 +559,7 @@ class BatchedBootstrapPF:
         return ll, ess, st
 
     def resample_threads(self, threads: int = 0):
-        """Threads per filter CTA of the resampler: pin 256, 512 or 1024, or
+        """Threads per CTA of the resampler: pin 256, 512 or 1024, or
         0 to keep the autotuned count; returns (current, {count: tuning us})."""
         cur = ctypes.c_int()
         us = np.zeros(3)
