@@ -53,8 +53,16 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t trow, const float* __re
   for (int n0 = 0; n0 < kProposalHidden; n0 += 16) {
     float v[16];
     tc::tmem_ld16(trow + (uint32_t)n0, v);
+    float4 b[4];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + __ldg(bias + n0 + j), 0.0f);
+    for (int j = 0; j < 4; ++j) b[j] = __ldg(reinterpret_cast<const float4*>(bias + n0) + j);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[4 * j] = fmaxf(v[4 * j] + b[j].x, 0.0f);
+      v[4 * j + 1] = fmaxf(v[4 * j + 1] + b[j].y, 0.0f);
+      v[4 * j + 2] = fmaxf(v[4 * j + 2] + b[j].z, 0.0f);
+      v[4 * j + 3] = fmaxf(v[4 * j + 3] + b[j].w, 0.0f);
+    }
     *reinterpret_cast<uint4*>(sOut + tc::kmajor_off(r, n0, kProposalHidden)) = pack8(v);
     *reinterpret_cast<uint4*>(sOut + tc::kmajor_off(r, n0 + 8, kProposalHidden)) = pack8(v + 8);
   }
