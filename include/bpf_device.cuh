@@ -31,7 +31,10 @@ namespace bpf {
 // launched without the attribute).  pdl_trigger() lets the next such kernel
 // be scheduled early; it is launched once every block of this kernel has
 // triggered or exited, and still waits in pdl_wait() for this kernel to
-// complete.
+// complete.  Such a kernel's lifetime overlaps its predecessors', so it reads
+// what they write with plain loads: the read-only path (__ldg, a const
+// __restrict__ parameter) is for data that nothing writes while a kernel
+// runs, such as observations, tables and weights.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -279,8 +282,9 @@ __device__ __forceinline__ bool transition_reduce_tail(LwPartial part, LwPartial
 }
 
 
-// Launch a kernel with the programmatic stream serialization attribute (its
-// body starts with pdl_wait()).
+// Launch a kernel with the programmatic stream serialization attribute.  Its
+// body calls pdl_wait() before it reads or writes anything that a kernel
+// before it uses; draws and constants may come earlier.
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args... args) {

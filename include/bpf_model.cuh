@@ -668,11 +668,11 @@ struct ModelStepArgs {
 template <class B> constexpr int state_columns() { return B::ND + B::NDX; }
 
 template <class B, class T>
-__device__ __forceinline__ void load_particle(ParticleVars<B, T>& v, const T* __restrict__ x, int ld, int src) {
+__device__ __forceinline__ void load_particle(ParticleVars<B, T>& v, const T* x, int ld, int src) {
 #pragma unroll
-  for (int j = 0; j < B::ND; ++j) v.d[j] = __ldg(x + (size_t)j * ld + src);
+  for (int j = 0; j < B::ND; ++j) v.d[j] = x[(size_t)j * ld + src];
 #pragma unroll
-  for (int j = 0; j < B::NDX; ++j) v.dx[j] = __ldg(x + (size_t)(B::ND + j) * ld + src);
+  for (int j = 0; j < B::NDX; ++j) v.dx[j] = x[(size_t)(B::ND + j) * ld + src];
 }
 
 template <class B, class T>

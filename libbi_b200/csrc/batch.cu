@@ -89,7 +89,7 @@ __global__ void k_batch_pz_init(T* x, int ld, double* lw, const BatchFilter* fil
 // ---------------------------------------------------------------------------
 template <class T, int D>
 __global__ void __launch_bounds__(kL96Block, l96_min_blocks(sizeof(T)))
-k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
+k_batch_l96_transition(const T* x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
                        double* __restrict__ lw, const T* __restrict__ y, double t1d, double t2d, int step,
                        const BatchFilter* __restrict__ filt, const L96Params* __restrict__ prms,
                        const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
@@ -109,7 +109,7 @@ k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld
     const int src = resampled ? min(max(as[col], 0), fd.n - 1) : p;
     T x0[D];
 #pragma unroll
-    for (int i = 0; i < D; ++i) x0[i] = __ldg(x_in + (size_t)i * ld + fd.off + src);
+    for (int i = 0; i < D; ++i) x0[i] = x_in[(size_t)i * ld + fd.off + src];
     l96_rk4<T, D>(x0, t1d, t2d, (T)prms[f].F, (T)prms[f].h);
 #pragma unroll
     for (int i = 0; i < D; ++i) sx[i][threadIdx.x] = x0[i];
@@ -133,7 +133,7 @@ k_batch_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld
 // filters' k_l96_transition_pair.
 template <class T, int D, int MB>
 __global__ void __launch_bounds__(2 * kL96Block, MB)
-k_batch_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
+k_batch_l96_transition_pair(const T* x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
                             double* __restrict__ lw, const T* __restrict__ y, double t1d, double t2d, int step,
                             const BatchFilter* __restrict__ filt, const L96Params* __restrict__ prms,
                             const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
@@ -171,7 +171,7 @@ k_batch_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, i
 
 template <class T>
 __global__ void __launch_bounds__(kPZBlock)
-k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
+k_batch_pz_transition(const T* x_in, T* __restrict__ x_out, int ld, int* __restrict__ as,
                       double* __restrict__ lw, const T* __restrict__ y, double t1d, double t2d, int step,
                       const BatchFilter* __restrict__ filt, const PZParams* __restrict__ prms,
                       const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
@@ -188,7 +188,7 @@ k_batch_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld,
   if (ok && p < fd.n) {
     const int col = fd.off + p;
     const int src = resampled ? min(max(as[col], 0), fd.n - 1) : p;
-    T P = __ldg(x_in + fd.off + src), Z = __ldg(x_in + (size_t)ld + fd.off + src);
+    T P = x_in[fd.off + src], Z = x_in[(size_t)ld + fd.off + src];
     const T alpha = pz_alpha<T>(fd.seed, (uint32_t)p, step, prm);
     pz_advance<T>(P, Z, alpha, t1d, t2d, prm);
     double l = resampled ? st->ll : lw[col];

@@ -179,7 +179,7 @@ inline int smem_bytes(int max_n, int G, bool mult) {
 // the loops took longer (14.2 against 12.6 us at N = 4096 on one CTA).
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT)
-k_batch_resample(const double* __restrict__ lw, int* __restrict__ as, const BatchFilter* __restrict__ sorted,
+k_batch_resample(const double* lw, int* __restrict__ as, const BatchFilter* __restrict__ sorted,
                  const int* __restrict__ order, StepStats* stats, double* lu_buf, int* os_buf, int step,
                  int G, int slot_bytes) {
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -200,7 +200,7 @@ k_batch_resample(const double* __restrict__ lw, int* __restrict__ as, const Batc
   const double* lwf = lw + fd.off;
   const int chunk = chunk_of(n, G);
   const int begin = min(n, rank * chunk), cn = min(n, begin + chunk) - begin;
-  double nx = tid < cn ? __ldg(lwf + begin + tid) : 0.0;
+  double nx = tid < cn ? lwf[begin + tid] : 0.0;
   if (st->resample == 0 || st->status != BPF_OK) return;  // uniform over the cluster
   // the cluster's CTAs may write to each other's shared memory once all of
   // them run: arrive here, wait before the first such write
@@ -230,7 +230,7 @@ k_batch_resample(const double* __restrict__ lw, int* __restrict__ as, const Batc
 #pragma unroll 1
       for (int l = tid; l < cn; l += NT) {
         const double x = nx;
-        if (l + NT < cn) nx = __ldg(lwf + begin + l + NT);
+        if (l + NT < cn) nx = lwf[begin + l + NT];
         const double d = __dsub_rn(x, mx);
         unsigned long long q = 0ull;
         if (!(d < kZeroBelow)) q = weight_to_fixed(nanexp(d));

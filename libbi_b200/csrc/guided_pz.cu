@@ -198,15 +198,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_pz_net(PZNetArgs a) {
       const int p = (blk - a.filt[nf_].block0) * kGTile + r;
       nlive = p < n;
       ncol = noff + p;
-      if (nlive) nsrc = a.stats[nf_].resample ? min(max(__ldg(a.as + ncol), 0), n - 1) : p;
+      if (nlive) nsrc = a.stats[nf_].resample ? min(max(a.as[ncol], 0), n - 1) : p;
     }
   };
   // stage 2: its state; stage 3: its features
   double nP = 1.0, nZ = 1.0;
   auto stage2 = [&]() {
     if (nlive) {
-      nP = __ldg(a.x_in + noff + nsrc);
-      nZ = __ldg(a.x_in + (size_t)a.ld + noff + nsrc);
+      nP = a.x_in[noff + nsrc];
+      nZ = a.x_in[(size_t)a.ld + noff + nsrc];
     }
   };
   float nu[3] = {0.0f, 0.0f, 0.0f};
@@ -273,11 +273,11 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_pz_net(PZNetArgs a) {
 // the step: proposal draw, ODE, observation and weight correction, per
 // filter reduction tail (the batched PZ transition's layout)
 __global__ void __launch_bounds__(kPZBlock)
-k_batch_pz_guided(const double* __restrict__ x_in, double* __restrict__ x_out, int ld, int* __restrict__ as,
+k_batch_pz_guided(const double* x_in, double* __restrict__ x_out, int ld, int* __restrict__ as,
                   double* __restrict__ lw, const double* __restrict__ y, double t1d, double t2d, int step,
                   const BatchFilter* __restrict__ filt, const PZParams* __restrict__ prms,
                   const int* __restrict__ blk2f, StepStats* stats, LwPartial* partials, unsigned* counters,
-                  double* hist, int nf, int k, const float2* __restrict__ O) {
+                  double* hist, int nf, int k, const float2* O) {
   pdl_wait();  // the network's outputs
   const int f = __ldg(blk2f + blockIdx.x);
   const BatchFilter fd = filt[f];
@@ -290,7 +290,7 @@ k_batch_pz_guided(const double* __restrict__ x_in, double* __restrict__ x_out, i
   if (ok && p < fd.n) {
     const int col = fd.off + p;
     const int src = resampled ? min(max(as[col], 0), fd.n - 1) : p;
-    double P = __ldg(x_in + fd.off + src), Z = __ldg(x_in + (size_t)ld + fd.off + src);
+    double P = x_in[fd.off + src], Z = x_in[(size_t)ld + fd.off + src];
     const float2 o = O[col];
     const double delta = (double)o.x;
     const double s = (double)fminf(fmaxf(o.y, kSMin), kSMax);

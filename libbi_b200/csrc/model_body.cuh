@@ -267,7 +267,7 @@ __device__ __forceinline__ void l96_pair_draw(T (&sz)[D / 2][2 * kL96Block], uin
 // to column p of x_out; the observation terms take the draws' place.  Every
 // thread of the block calls it (the halves meet in shuffles).
 template <class T, int D>
-__device__ __forceinline__ void l96_pair_step(T (&sz)[D / 2][2 * kL96Block], const T* __restrict__ x_in, int src,
+__device__ __forceinline__ void l96_pair_step(T (&sz)[D / 2][2 * kL96Block], const T* x_in, int src,
                                               T* __restrict__ x_out, int p, int ld, bool live,
                                               const T* __restrict__ y, uint64_t mask, double t1d, double t2d,
                                               const L96Params& prm) {
@@ -277,7 +277,7 @@ __device__ __forceinline__ void l96_pair_step(T (&sz)[D / 2][2 * kL96Block], con
   const int tid = threadIdx.x, c0 = (tid & 1) * H;
   T x0[H];
 #pragma unroll
-  for (int i = 0; i < H; ++i) x0[i] = live ? __ldg(x_in + (size_t)(c0 + i) * ld + src) : (T)0;
+  for (int i = 0; i < H; ++i) x0[i] = live ? x_in[(size_t)(c0 + i) * ld + src] : (T)0;
   l96_rk4_half<T, H>(x0, t1d, t2d, (T)prm.F, (T)prm.h);
   if (!live) return;
   const T se = (T)prm.sigma_eta;

@@ -20,7 +20,7 @@ namespace bpf {
 
 template <class T, int D>
 __global__ void __launch_bounds__(kL96Block, l96_min_blocks(sizeof(T)))
-k_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n,
+k_l96_transition(const T* x_in, T* __restrict__ x_out, int ld, int n,
                  int* __restrict__ as, double* __restrict__ lw, const T* __restrict__ y,
                  double t1d, double t2d, uint64_t seed, int step, L96Params prm,
                  StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask) {
@@ -35,7 +35,7 @@ k_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int 
     const int src = resampled ? as[p] : p;
     T x0[D];
 #pragma unroll
-    for (int i = 0; i < D; ++i) x0[i] = __ldg(x_in + (size_t)i * ld + src);
+    for (int i = 0; i < D; ++i) x0[i] = x_in[(size_t)i * ld + src];
     l96_rk4<T, D>(x0, t1d, t2d, (T)prm.F, (T)prm.h);
 #pragma unroll
     for (int i = 0; i < D; ++i) sx[i][threadIdx.x] = x0[i];
@@ -55,7 +55,7 @@ k_l96_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int 
 // on an SM.
 template <class T, int D, int MB>
 __global__ void __launch_bounds__(2 * kL96Block, MB)
-k_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n,
+k_l96_transition_pair(const T* x_in, T* __restrict__ x_out, int ld, int n,
                       int* __restrict__ as, double* __restrict__ lw, const T* __restrict__ y,
                       double t1d, double t2d, uint64_t seed, int step, L96Params prm,
                       StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask) {
@@ -85,7 +85,7 @@ k_l96_transition_pair(const T* __restrict__ x_in, T* __restrict__ x_out, int ld,
 
 template <class T>
 __global__ void __launch_bounds__(kPZBlock)
-k_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n,
+k_pz_transition(const T* x_in, T* __restrict__ x_out, int ld, int n,
                 int* __restrict__ as, double* __restrict__ lw, const T* __restrict__ y,
                 double t1d, double t2d, uint64_t seed, int step, PZParams prm,
                 StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask) {
@@ -98,7 +98,7 @@ k_pz_transition(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n
   LwPartial part = lw_empty();
   if (p < n && ok) {
     const int src = resampled ? as[p] : p;
-    T P = __ldg(x_in + src), Z = __ldg(x_in + (size_t)ld + src);
+    T P = x_in[src], Z = x_in[(size_t)ld + src];
     pz_advance<T>(P, Z, alpha, t1d, t2d, prm);
     double l = resampled ? st->ll : lw[p];
     if (y && (mask & 1ull)) l += pz_obs_term<T>(P, __ldg(y), prm);

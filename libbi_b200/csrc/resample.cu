@@ -881,13 +881,13 @@ k_systematic_coop(const double* __restrict__ lw, int n, StepStats* st, const dou
 // integers (the shape is chosen by the autotuner below).
 // IT log-weights of one thread (16-byte loads when IT is even and aligned)
 template <int IT>
-__device__ __forceinline__ void load_items(const double* __restrict__ lw, int i0, int n, double (&v)[IT]) {
+__device__ __forceinline__ void load_items(const double* lw, int i0, int n, double (&v)[IT]) {
   if constexpr (IT % 2 == 0) {
     if (i0 + IT <= n && ((reinterpret_cast<uintptr_t>(lw + i0) & 15) == 0)) {
       const double2* p = reinterpret_cast<const double2*>(lw + i0);
 #pragma unroll
       for (int k = 0; k < IT / 2; ++k) {
-        const double2 t = __ldg(p + k);
+        const double2 t = p[k];
         v[2 * k] = t.x;
         v[2 * k + 1] = t.y;
       }
@@ -895,12 +895,12 @@ __device__ __forceinline__ void load_items(const double* __restrict__ lw, int i0
     }
   }
 #pragma unroll
-  for (int k = 0; k < IT; ++k) v[k] = (i0 + k < n) ? __ldg(lw + i0 + k) : NAN;
+  for (int k = 0; k < IT; ++k) v[k] = (i0 + k < n) ? lw[i0 + k] : NAN;
 }
 
 template <int NT, int IT>
 __global__ void __launch_bounds__(NT)
-k_systematic_coop1(const double* __restrict__ lw, int n, StepStats* st, const double* a_in, uint64_t seed,
+k_systematic_coop1(const double* lw, int n, StepStats* st, const double* a_in, uint64_t seed,
                    int step, int* Os_out, int* as, int* E, int* ecoarse, int coarse_shift, int* slot,
                    unsigned long long* pub, int pub_stride, unsigned* epoch_word, const int* gate) {
   // the next kernel (the transition, a programmatic dependent) may be

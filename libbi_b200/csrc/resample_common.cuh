@@ -117,7 +117,7 @@ __device__ __forceinline__ bool metropolis_accept(uint32_t hi, uint32_t lo, doub
 // (share/src/bi/host/resampler/MetropolisResamplerHost.hpp:290-321); draw k
 // uses (u_int, u_acc) = u[2(p*B+k)], u[2(p*B+k)+1] when u is given, else the
 // counter-based stream.
-__device__ __forceinline__ int metropolis_ancestor(const double* __restrict__ lw, int n, int B, const double* u,
+__device__ __forceinline__ int metropolis_ancestor(const double* lw, int n, int B, const double* u,
                                                    uint64_t seed, int step, int p) {
   const double nd = (double)n;
   int p1 = p;
@@ -134,7 +134,7 @@ __device__ __forceinline__ int metropolis_ancestor(const double* __restrict__ lw
     int p2 = __double2int_rz(__dmul_rn(ui, nd));
     p2 = p2 < n - 1 ? p2 : n - 1;  // uniformInt(0, n-1); also bounds caller-supplied uniforms
     p2 = p2 > 0 ? p2 : 0;
-    double lw2 = __ldg(lw + p2);
+    double lw2 = lw[p2];
     const double d = __dsub_rn(lw2, lw1);
     if (u ? log(u[2 * ((size_t)p * B + k) + 1]) < d : metropolis_accept(r.v[2], r.v[3], d)) {
       p1 = p2;

@@ -42,7 +42,7 @@ constexpr int kFusedMaxBlocks = 8 * kL96Block;
 // over the launch's blocks (every block calls it; false: a wait gave up or
 // the weights were degenerate, recorded in the status)
 template <int NT>
-__device__ __noinline__ bool fused_systematic_ancestor(const double* __restrict__ lw, int n, StepStats* st,
+__device__ __noinline__ bool fused_systematic_ancestor(const double* lw, int n, StepStats* st,
                                                           uint64_t seed, int step, int* __restrict__ E,
                                                           int* __restrict__ ecoarse, unsigned long long* pub,
                                                           unsigned* epoch_word, long long lim, int* s_coarse,
@@ -61,7 +61,7 @@ __device__ __noinline__ bool fused_systematic_ancestor(const double* __restrict_
 
   // 1. the particle's fixed-point weight and the block total
   u128 qq;
-  qq.lo = live ? weight_to_fixed(nanexp(__dsub_rn(__ldg(lw + p), mx))) : 0ull;
+  qq.lo = live ? weight_to_fixed(nanexp(__dsub_rn(lw[p], mx))) : 0ull;
   qq.hi = 0;
   u128 btot;
   const u128 texcl = block_exclusive_scan_u128_nt<NT>(qq, &btot);
@@ -189,7 +189,7 @@ __device__ __noinline__ bool fused_systematic_ancestor(const double* __restrict_
 // it is k_l96_transition; with it, the prologue above first.
 template <class T, int D>
 __global__ void __launch_bounds__(kL96Block, l96_min_blocks(sizeof(T)))
-k_l96_step(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n, int* __restrict__ as,
+k_l96_step(const T* x_in, T* __restrict__ x_out, int ld, int n, int* __restrict__ as,
            double* __restrict__ lw, const T* __restrict__ y, double t1d, double t2d, uint64_t seed, int step,
            L96Params prm, StepStats* st, LwPartial* partials, unsigned* counter, uint64_t mask, int* E,
            int* ecoarse, unsigned long long* pub, unsigned* epoch_word, long long lim) {
@@ -207,7 +207,7 @@ k_l96_step(const T* __restrict__ x_in, T* __restrict__ x_out, int ld, int n, int
   if (ok && p < n) {
     T x0[D];
 #pragma unroll
-    for (int i = 0; i < D; ++i) x0[i] = __ldg(x_in + (size_t)i * ld + src);
+    for (int i = 0; i < D; ++i) x0[i] = x_in[(size_t)i * ld + src];
     l96_rk4<T, D>(x0, t1d, t2d, (T)prm.F, (T)prm.h);
 #pragma unroll
     for (int i = 0; i < D; ++i) sx[i][threadIdx.x] = x0[i];

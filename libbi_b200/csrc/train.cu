@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(64) k_reduce_adam(ReduceAdamArgs a) {
   if (blockIdx.x == gridDim.x - 1) {
     if (threadIdx.x < 32) {
       double t = 0.0;
-      for (int k = threadIdx.x; k < a.tiles; k += 32) t += __ldcg(a.loss_part + k);
+      for (int k = threadIdx.x; k < a.tiles; k += 32) t += a.loss_part[k];
       t = warp_sum(t);
       if (threadIdx.x == 0) *a.loss = t / (double)a.B;
     }
@@ -425,12 +425,12 @@ __global__ void __launch_bounds__(64) k_reduce_adam(ReduceAdamArgs a) {
   for (; k + 32 <= terms; k += 32) {
     float v[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __ldcg(src + (k + j) * stride);
+    for (int j = 0; j < 32; ++j) v[j] = src[(k + j) * stride];
 #pragma unroll
     for (int j = 0; j < 32; ++j) g += v[j];
   }
 #pragma unroll 4
-  for (; k < terms; ++k) g += __ldcg(src + k * stride);
+  for (; k < terms; ++k) g += src[k * stride];
   a.grads[i] = g;
   if (!a.P) return;
   // rounded as k_adam's expressions are compiled (proposal.cu), so that a run
