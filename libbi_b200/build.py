@@ -38,7 +38,8 @@ def up_to_date() -> bool:
     if not os.path.exists(OUT):
         return False
     t = os.path.getmtime(OUT)
-    deps = sources() + glob.glob(os.path.join(SRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    headers = [os.path.join(d, e) for d in (SRC, os.path.join(HERE, "..", "include")) for e in ("*.h", "*.cuh")]
+    deps = sources() + [f for pattern in headers for f in glob.glob(pattern)]
     return all(os.path.getmtime(d) <= t for d in deps)
 
 

@@ -11,6 +11,7 @@
 #include "proposal.cuh"
 #include "batch.cuh"
 #include "resample_common.cuh"
+#include "host_slots.h"
 
 #include <cstdio>
 #include <map>
@@ -100,9 +101,7 @@ struct bpf_resampler {
   int shape = -1;  // pinned tile shape of the one-launch systematic kernel
   cudaStream_t stream = nullptr;
   bpf::ResampleScratch rs;
-  // pinned copy of the statistics: 4.5 us less per reduction and resampling
-  // (62.1 -> 57.6 us at 1000 particles) for some 2.7 ms when a handle is made
-  bpf::StepStats* host_stats = nullptr;
+  bpf::StepStats* host_stats = nullptr;  // pinned copy of the statistics, or null (g_host_stats)
   // optional device timing of the compute kernels of each call (events
   // after the status reset and before the read-back)
   bool timing = false;
@@ -1049,6 +1048,21 @@ int bpf_timing_read(bpf_handle* h, int reset, double* resample_ms, double* trans
 
 // ---- stand-alone resampler ------------------------------------------------
 
+// where the stand-alone resamplers' statistics are read back to (one page)
+static void* pin_block(size_t bytes) {
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+static bool block_is_pinned(void* block) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, block) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+static bpf::HostSlots<bpf::StepStats, (int)(4096 / sizeof(bpf::StepStats))> g_host_stats(pin_block, block_is_pinned);
+
 int bpf_resampler_create(int kind, int max_n, int metropolis_steps, void* stream, bpf_resampler** out) {
   if (!out) return BPF_E_INVALID;
   *out = nullptr;
@@ -1061,10 +1075,7 @@ int bpf_resampler_create(int kind, int max_n, int metropolis_steps, void* stream
   r->stream = (cudaStream_t)stream;
   int rc = bpf::scratch_alloc(r->rs, max_n);
   if (rc) { delete r; return rc; }
-  if (cudaMallocHost((void**)&r->host_stats, sizeof(bpf::StepStats)) != cudaSuccess) {
-    cudaGetLastError();
-    r->host_stats = nullptr;  // read back through pageable memory instead
-  }
+  r->host_stats = g_host_stats.acquire();
   *out = r;
   return BPF_OK;
 }
@@ -1074,7 +1085,7 @@ int bpf_resampler_destroy(bpf_resampler* r) {
   if (r->stream) cudaStreamSynchronize(r->stream); else cudaDeviceSynchronize();
   for (cudaEvent_t e : r->ev)
     if (e) cudaEventDestroy(e);
-  if (r->host_stats) cudaFreeHost(r->host_stats);
+  g_host_stats.release(r->host_stats);
   bpf::scratch_free(r->rs);
   delete r;
   return BPF_OK;
@@ -1107,7 +1118,8 @@ static int timing_collect(bpf_resampler* r) {
 }
 
 static int read_rs_stats(bpf_resampler* r, bpf::StepStats* s) {
-  // through the handle's pinned copy: a direct DMA instead of a staged copy
+  // through the handle's pinned slot, if it has one: a direct DMA instead of a
+  // staged copy
   bpf::StepStats* dst = r->host_stats ? r->host_stats : s;
   BPF_TRY(cudaMemcpyAsync(dst, r->rs.stats, sizeof(*s), cudaMemcpyDeviceToHost, r->stream));
   BPF_TRY(cudaStreamSynchronize(r->stream));
