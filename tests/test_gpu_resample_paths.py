@@ -130,3 +130,33 @@ def test_stand_alone_resamplers_on_stressed_weights(cuda, oracle, n, offset):
             np.testing.assert_array_equal(got, permuted, err_msg=f"{kind} {pattern} permuted")
     for r in made.values():
         r.close()
+
+
+WIDE = 148 * 8 * 256  # slots that one block per 256 of them still holds at once
+
+
+@pytest.mark.parametrize("n", [2**18 - 1, 2**18, WIDE, WIDE + 1, 2**19 - 1, 2**19, 1000003])
+def test_stand_alone_resamplers_at_their_wide_forms(cuda, oracle, n):
+    """Both sides of the sizes from which a multinomial tile holds 4 and 8
+    particles per thread and a thread searches for four slots, and an odd size
+    well beyond them: the multinomial ancestors sorted and permuted, the
+    systematic ones sorted (permuted they take another kernel), the Metropolis
+    ones permuted (unpermuted ones need no search)."""
+    import torch
+    from libbi_b200 import MetropolisResampler, MultinomialResampler, SystematicResampler
+
+    made = {"multinomial": (MultinomialResampler(max_n=n), (False, True)),
+            "systematic": (SystematicResampler(max_n=n), (False,)),
+            "metropolis": (MetropolisResampler(max_n=n, B=B), (True,))}
+    rng = np.random.default_rng(n)
+    for pattern, lw in _patterns(n, n).items():
+        lw_d = torch.as_tensor(lw, device="cuda")
+        for kind, (r, forms) in made.items():
+            u = rng.random({"systematic": 1, "multinomial": n, "metropolis": 2 * n * B}[kind])
+            u_d = torch.as_tensor(u, device="cuda")
+            want = _want(oracle, kind, lw, u)
+            for permute in forms:
+                got = r.ancestors(lw_d, u_d, permute=permute).cpu().numpy()
+                np.testing.assert_array_equal(got, want[permute], err_msg=f"{kind} {pattern} permute={permute}")
+    for r, _ in made.values():
+        r.close()
