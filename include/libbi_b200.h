@@ -444,7 +444,8 @@ int bpf_batch_set_seeds(bpf_batch* b, const uint64_t* seeds);
  * log-weights laid out as the batch's filters and the fastest is kept; every
  * choice computes the same ancestors.  threads != 0 pins a count (a captured
  * filter run is recaptured); current and tuned_us[3] (the tuning times for
- * 256, 512, 1024 with the kept cluster size; may be NULL) report the state. */
+ * 256, 512, 1024 with the kept cluster size, infinite for a count that could
+ * not be launched; may be NULL) report the state. */
 int bpf_batch_resample_threads(bpf_batch* b, int threads, int* current, double* tuned_us);
 /* One BootstrapPF::step of every filter (see bpf_step); y_device: device
  * observations, nfilters x (dim for L96, 1 for PZ), filter-major, in the

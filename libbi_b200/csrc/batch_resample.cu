@@ -16,10 +16,10 @@
 #include "internal.cuh"
 #include "resample_common.cuh"
 #include "batch.cuh"
+#include "tune_pick.h"
 #include "../../include/bpf_math.h"
 
 #include <algorithm>
-#include <vector>
 
 namespace bpf {
 
@@ -549,7 +549,7 @@ __global__ void k_batch_tune_stats(const double* lw, const BatchFilter* filt, St
 // thread counts, on synthetic log-weights laid out as the batch's
 // filters (scratch buffers: the batch's own state is untouched), and put the
 // fastest into the plan; its cluster size's medians go to us[3] (256, 512,
-// 1024 threads).
+// 1024 threads; infinite for one that could not be launched).
 int tune_batch_resample(const BatchFilter* filt, ResamplePlan* p, int ld, cudaStream_t st, double* us) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   BPF_TRY(cudaStreamIsCapturing(st, &cs));
@@ -574,46 +574,38 @@ int tune_batch_resample(const BatchFilter* filt, ResamplePlan* p, int ld, cudaSt
     k_batch_tune_stats<<<p->nf, 256, 0, st>>>(lw, filt, stats, p->nf);
     if (cudaGetLastError() != cudaSuccess) rc = BPF_E_CUDA;
   }
-  // the candidates take turns, round after round, so that a drift of clocks
-  // or caches during the tuning reaches every one alike; medians decide, among
-  // those that the first round left within kNear of its best.  The first
-  // launch of each thread count, which loads its code, is not timed.
+  // candidates: every cluster size from the smallest that holds the largest
+  // filter, each with the three thread counts.  The first launch of each
+  // count, which loads its code, is not timed.
   constexpr int kReps = 3, kMax = 12;
   constexpr float kNear = 1.25f;
   ResamplePlan c[kMax];
-  float t[kMax][kReps], med[kMax];
-  bool in[kMax];
-  int nc = 0;
+  float med[kMax];
+  int nc = 0, best = -1;
   for (int g = p->group; g <= kGroup; g *= 2)
     for (int thr = 256; thr <= 1024; thr *= 2) {
       c[nc] = *p;
       c[nc].group = g;
-      c[nc].threads = thr;
-      in[nc++] = true;
+      c[nc++].threads = thr;
     }
-  for (int k = 0; !rc && k < 3; ++k) rc = launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st);
-  for (int r = 0; !rc && r < kReps; ++r) {
-    for (int k = 0; !rc && k < nc; ++k) {
-      if (!in[k]) continue;
-      if (cudaEventRecord(e0, st) != cudaSuccess) { rc = BPF_E_CUDA; break; }
-      rc = launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st);
-      if (!rc && (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-                  cudaEventElapsedTime(&t[k][r], e0, e1) != cudaSuccess))
-        rc = BPF_E_CUDA;
+  auto timed = [&](int k, float* ms) -> int {
+    if (cudaEventRecord(e0, st) != cudaSuccess) return BPF_E_CUDA;
+    const int e = launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st);
+    if (e) {
+      cudaGetLastError();  // this candidate's alone
+      return e;
     }
-    if (r == 0 && !rc) {
-      float least = t[0][0];
-      for (int k = 1; k < nc; ++k) least = std::min(least, t[k][0]);
-      for (int k = 0; k < nc; ++k) in[k] = t[k][0] <= kNear * least;
-    }
+    if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+        cudaEventElapsedTime(ms, e0, e1) != cudaSuccess)
+      return BPF_E_CUDA;
+    return BPF_OK;
+  };
+  if (!rc) {
+    for (int k = 0; k < 3; ++k)
+      if (launch_batch_resample(lw, as, c[k], stats, lu, os, 1, st)) cudaGetLastError();
+    rc = pick_fastest<kMax, kReps>(nc, kNear, timed, med, &best);
   }
   if (!rc) {
-    int best = -1;
-    for (int k = 0; k < nc; ++k) {
-      if (in[k]) std::sort(t[k], t[k] + kReps);
-      med[k] = t[k][in[k] ? kReps / 2 : 0];
-      if (in[k] && (best < 0 || med[k] < med[best])) best = k;
-    }
     *p = c[best];
     // the thread counts' times with the kept cluster size
     if (us)
