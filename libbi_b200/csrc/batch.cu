@@ -236,7 +236,7 @@ static int batch_l96_transition(const void* x_in, void* x_out, int ld, int* as, 
                                 int blocks, StepStats* stats, LwPartial* partials, unsigned* counters, double* hist,
                                 int nf, int k, cudaStream_t st) {
   if constexpr (D % 8 == 0) {
-    const int mb = l96_pair_blocks(sizeof(T), blocks);
+    const int mb = l96_pair_blocks(D, sizeof(T), blocks);
     if (mb == 2) {
       BATCH_L96_LAUNCH((k_batch_l96_transition_pair<T, D, 2>), 2 * kL96Block);
       return BPF_OK;
@@ -248,7 +248,7 @@ static int batch_l96_transition(const void* x_in, void* x_out, int ld, int* as, 
       }
     }
   }
-  if constexpr (D % 8 != 0 || sizeof(T) == 4) {
+  if constexpr (D < 32 || sizeof(T) == 4) {
     BATCH_L96_LAUNCH((k_batch_l96_transition<T, D>), kL96Block);
     return BPF_OK;
   }

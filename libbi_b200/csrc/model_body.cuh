@@ -19,6 +19,7 @@
 #include "reduce.cuh"
 #include "../../include/bpf_math.h"
 #include "f32x2.cuh"
+#include "l96_forms.h"
 
 #include <cmath>
 
@@ -233,21 +234,8 @@ __device__ __forceinline__ double l96_noise_obs(const T (&sx)[D][kL96Block], T* 
 // fourth cycle, the FP64 pipe 28 % busy), which this halves; the draws, which
 // need nothing of the kernel before, come before the wait for it.  Same
 // arithmetic, and one thread per particle adds its terms and enters the
-// reduction, so the same bits.
+// reduction, so the same bits.  Where this form is taken: l96_forms.h.
 // ---------------------------------------------------------------------------
-// Blocks of the two-thread form on an SM for a launch of `blocks` blocks, or 0
-// for one thread per particle.  Microseconds per filter step on B200 (d = 40,
-// resampler included), one thread / two threads: FP32 25.3 / 21.2 at N = 4096,
-// 31.7 / 27.1 at 18944, 37.6 / 30.3 at 37888 (two blocks on every SM; 36.6
-// compiled for three), 44.3 / 38.0 at 56832 (three), 44.4 / 46.7 at 65536 (a
-// second wave); FP64 33.8 / 24.8 at 4096, 40.8 / 33.9 at 20011, 69.1 / 60.8 at
-// 65536, 699 / 643 at 10^6: there one thread's 255 registers leave an SM half
-// the warps at any size.
-inline int l96_pair_blocks(int esz, int blocks) {
-  if (esz == 8) return 2;
-  return blocks <= 2 * 148 ? 2 : blocks <= 3 * 148 ? 3 : 0;
-}
-
 // the thread's draws, by component
 template <class T, int D>
 __device__ __forceinline__ void l96_pair_draw(T (&sz)[D / 2][2 * kL96Block], uint64_t seed, uint32_t prng, int step) {

@@ -162,7 +162,7 @@ template <class T, int D>
 static int l96_transition(const ModelArgs& m, const TransitionArgs& a, int blocks, cudaStream_t st) {
   const L96Params prm = l96_params<T>(m.theta, m.h);
   if constexpr (D % 8 == 0) {
-    const int mb = l96_pair_blocks(sizeof(T), blocks);
+    const int mb = l96_pair_blocks(D, sizeof(T), blocks);
     if (mb == 2) {
       L96_LAUNCH((k_l96_transition_pair<T, D, 2>), 2 * kL96Block);
       return BPF_OK;
@@ -174,7 +174,7 @@ static int l96_transition(const ModelArgs& m, const TransitionArgs& a, int block
       }
     }
   }
-  if constexpr (D % 8 != 0 || sizeof(T) == 4) {
+  if constexpr (D < 32 || sizeof(T) == 4) {
     L96_LAUNCH((k_l96_transition<T, D>), kL96Block);
     return BPF_OK;
   }

@@ -12,6 +12,7 @@ CASES = [(dim, prec, n) for dim in (8, 16, 32, 40) for prec in ("f32", "f64") fo
 CASES += [(4, "f64", BLOCK + 1)]
 CASES += [(40, "f32", 2 * 148 * BLOCK + i) for i in (0, 1)] + [(40, "f32", 3 * 148 * BLOCK + i) for i in (0, 1)]
 CASES += [(40, "f64", 2 * 148 * BLOCK + 1)]
+CASES += [(dim, "f64", 2 * 148 * BLOCK + i) for dim in (8, 16) for i in (0, 1)]
 
 
 def _want(oracle, model, n, seed, y, T, dt):

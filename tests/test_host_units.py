@@ -8,7 +8,7 @@ import pytest
 CPP = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp")
 
 
-@pytest.mark.parametrize("name", ["host_slots", "tune_pick"])
+@pytest.mark.parametrize("name", ["host_slots", "tune_pick", "l96_forms"])
 def test_host_unit(name, tmp_path):
     exe = str(tmp_path / name)
     subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-Wall", "-Werror", os.path.join(CPP, name + "_test.cpp"),
