@@ -359,7 +359,7 @@ int ProposalNet::alloc(int d, int hid, int cap_batch, int din_) {
   if (!rc) rc = A((void**)&r0, (size_t)cap * dim * 4);
   if (l96) {
     // the shares of the weight gradients, the bias sums and the losses
-    ws_floats = (long long)kTrainMaxShares * nparams;
+    ws_floats = (long long)train_shares(cap) * nparams;
     if (!rc) rc = A((void**)&ws, (size_t)ws_floats * 4);
     if (!rc) rc = A((void**)&colpart, (size_t)train_colpart_floats(cap) * 4);
     if (!rc) rc = A((void**)&loss_part, (size_t)((cap + 127) / 128) * sizeof(double));

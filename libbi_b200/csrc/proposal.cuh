@@ -88,6 +88,7 @@ struct TrainBatch {
 };
 // CTAs, and so shares of the weight gradients, at most: one per SM
 constexpr int kTrainMaxShares = 148;
+int train_shares(int B);  // CTAs of a minibatch of B rows
 long long train_colpart_floats(int cap);
 int launch_train_tile(ProposalNet& p, const TrainBatch& t, cudaStream_t st);
 // the gradient into ProposalNet::grads, the mean loss to *loss (device), and

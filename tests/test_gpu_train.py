@@ -71,3 +71,19 @@ def test_unaligned_data_trains_alike(cuda, offset):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
     assert np.isfinite(out[0][0]).all() and (out[0][1] != P0).any()
+
+
+def test_workspace_follows_the_capacity(cuda):
+    """Eight proposals for batches of 128 rows, one share of the gradient each
+    (147 KB): far less device memory than the 148 shares of a full GPU (22 MB
+    each)."""
+    import torch
+    from libbi_b200 import LearnedProposal, ModelL96
+
+    LearnedProposal(ModelL96(dim=40), 0.05, 128, 1).close()
+    free0 = torch.cuda.mem_get_info()[0]
+    made = [LearnedProposal(ModelL96(dim=40), 0.05, 128, 1) for _ in range(8)]
+    used = free0 - torch.cuda.mem_get_info()[0]
+    for p in made:
+        p.close()
+    assert used <= 8 * (4 << 20), used
