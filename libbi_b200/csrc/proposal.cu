@@ -355,6 +355,7 @@ int ProposalNet::alloc(int d, int hid, int cap_batch, int din_) {
   if (!rc) rc = A((void**)&scale, (size_t)din * 4);
   if (!rc) rc = A((void**)&err, sizeof(int));
   if (!rc) rc = A((void**)&loss, sizeof(double));
+  if (!rc) rc = A((void**)&losses, kLossChunk * sizeof(double));
   if (!rc) rc = A((void**)&U, (size_t)cap * din * 2);
   if (!rc) rc = A((void**)&r0, (size_t)cap * dim * 4);
   if (l96) {
@@ -576,18 +577,8 @@ int bpf_proposal_train(bpf_proposal* q, int steps, int batch, double lr, float* 
   // learning rate: linear warm-up over the first 5% of the steps, then a
   // cosine decay to a tenth
   const int warm = steps / 20 > 1 ? steps / 20 : 1;
-  // the steps' losses stay on the device until the last one is enqueued
-  if (steps > p.losses_cap) {
-    if (p.losses) cudaFree(p.losses);
-    p.losses = nullptr;
-    p.losses_cap = 0;
-    if (cudaMalloc((void**)&p.losses, (size_t)steps * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return BPF_E_NOMEM;
-    }
-    p.losses_cap = steps;
-  }
   for (int s = 0; s < steps; ++s) {
+    const int slot = s % bpf::kLossChunk;  // of this step's loss
     const double w = s < warm ? (double)(s + 1) / warm : 1.0;
     const double c = 0.1 + 0.9 * 0.5 * (1.0 + std::cos(3.14159265358979323846 * s / (double)steps));
     const double lr_s = lr * w * c;
@@ -612,20 +603,22 @@ int bpf_proposal_train(bpf_proposal* q, int steps, int batch, double lr, float* 
     ++q->train_step;
     const float c1 = 1.0f - std::pow(b1, (float)q->adam_step), c2 = 1.0f - std::pow(b2, (float)q->adam_step);
     if (p.l96) {
-      rc = bpf::launch_reduce_adam(p, batch, p.losses + s, true, (float)lr_s, b1, b2, eps, c1, c2, q->stream);
+      rc = bpf::launch_reduce_adam(p, batch, p.losses + slot, true, (float)lr_s, b1, b2, eps, c1, c2, q->stream);
       if (rc) return rc;
     } else {
       bpf::k_adam<<<(p.nparams + 255) / 256, 256, 0, q->stream>>>(p.params, p.grads, p.m1, p.m2, p.params_h,
                                                                  p.nparams, (float)lr_s, b1, b2, eps, c1, c2);
       BPF_TRY(cudaGetLastError());
-      BPF_TRY(cudaMemcpyAsync(p.losses + s, p.loss, sizeof(double), cudaMemcpyDeviceToDevice, q->stream));
+      BPF_TRY(cudaMemcpyAsync(p.losses + slot, p.loss, sizeof(double), cudaMemcpyDeviceToDevice, q->stream));
     }
-  }
-  if (loss_trace && steps > 0) {
-    std::vector<double> l((size_t)steps);
-    BPF_TRY(cudaMemcpyAsync(l.data(), p.losses, l.size() * sizeof(double), cudaMemcpyDeviceToHost, q->stream));
-    BPF_TRY(cudaStreamSynchronize(q->stream));
-    for (int s = 0; s < steps; ++s) loss_trace[s] = (float)l[s];
+    // the losses stay on the device until a chunk of steps, or the last step,
+    // is enqueued: one synchronisation for all of them
+    if (loss_trace && (slot == bpf::kLossChunk - 1 || s == steps - 1)) {
+      double l[bpf::kLossChunk];
+      BPF_TRY(cudaMemcpyAsync(l, p.losses, (size_t)(slot + 1) * sizeof(double), cudaMemcpyDeviceToHost, q->stream));
+      BPF_TRY(cudaStreamSynchronize(q->stream));
+      for (int k = 0; k <= slot; ++k) loss_trace[s - slot + k] = (float)l[k];
+    }
   }
   if (!p.l96) {  // the two-launch step keeps the images current
     const int rc = bpf::pack_weights(p, q->stream);

@@ -17,6 +17,10 @@ constexpr float kSMin = -7.0f, kSMax = 3.0f;
 // the activations
 constexpr int kPZNetK1 = 16, kPZNetK2 = kProposalHidden + 16, kPZNetN3 = 16;
 
+// steps of a training call whose losses stay on the device before they are
+// read back
+constexpr int kLossChunk = 1024;
+
 struct ProposalNet {
   // dim: the proposed variables (the L96 state's 40 components; the PZ
   // model's one log-noise), din: network inputs, dout = 2 dim: (delta, s)
@@ -56,8 +60,7 @@ struct ProposalNet {
   float* ws = nullptr;       // shares (L96: per tile) or split-K parts of the weight gradients
   long long ws_floats = 0;
   double* loss_part = nullptr;  // per-block loss sums
-  double* losses = nullptr;     // losses of a training call's steps
-  int losses_cap = 0;
+  double* losses = nullptr;     // the latest losses of a training call's steps (kLossChunk)
 
   const __nv_bfloat16* w1h() const { return params_h + o_w1; }
   const __nv_bfloat16* w2h() const { return params_h + o_w2; }

@@ -87,3 +87,32 @@ def test_workspace_follows_the_capacity(cuda):
     for p in made:
         p.close()
     assert used <= 8 * (4 << 20), used
+
+
+def test_long_traces_are_whole_and_take_no_memory(cuda):
+    """At a learning rate far below every parameter's rounding (a zero weight
+    moves to 1e-30) a step's loss depends on its minibatch alone, and minibatches follow the count of steps: the trace
+    of one long call equals those of shorter ones, across the read-backs of
+    1024 steps.  A call's device memory does not grow with its steps (300 000
+    losses would take 2.4 MB)."""
+    import torch
+    from libbi_b200 import LearnedProposal, ModelL96
+
+    data = _data(500, 11)
+
+    def made():
+        p = LearnedProposal(ModelL96(dim=40), 0.05, 128, 5)
+        p.set_data(*data)
+        return p
+
+    p, q = made(), made()
+    got = p.train(2600, 16, 1e-30)
+    want = np.concatenate([q.train(n, 16, 1e-30) for n in (1, 1023, 1024, 552)])
+    assert np.isfinite(got).all()
+    np.testing.assert_array_equal(got, want)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    p.train(300000, 1, 1e-30)
+    assert free0 - torch.cuda.mem_get_info()[0] < 1 << 20
+    p.close()
+    q.close()
