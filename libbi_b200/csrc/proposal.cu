@@ -507,6 +507,7 @@ int bpf_proposal_set_states(bpf_proposal* q, const double* x_t, int n) {
   if (p.target) cudaFree(p.target);
   p.feat = p.target = nullptr;
   p.rows = 0;
+  q->n = 0;  // nothing to train on until the new rows are there
   if (cudaMalloc((void**)&p.feat, (size_t)n * p.din * 4) != cudaSuccess ||
       cudaMalloc((void**)&p.target, (size_t)n * p.dim * 4) != cudaSuccess) {
     cudaGetLastError();
@@ -541,6 +542,7 @@ int bpf_proposal_set_data(bpf_proposal* q, const float* x_t, const float* x_t1, 
   bpf::ProposalNet& p = q->net;
   if (p.mt) cudaFree(p.mt);
   p.mt = nullptr;
+  q->n = 0;  // nothing to train on until the new rows are there
   if (cudaMalloc((void**)&p.mt, (size_t)n * p.dim * 4) != cudaSuccess) { cudaGetLastError(); return BPF_E_NOMEM; }
   q->xt = x_t; q->xt1 = x_t1; q->yt1 = y_t1; q->n = n;
   bpf::k_rk4_mean<40><<<(n + 127) / 128, 128, 0, q->stream>>>(x_t, p.mt, n, q->dt, q->model.theta[0], q->model.h);

@@ -116,3 +116,20 @@ def test_long_traces_are_whole_and_take_no_memory(cuda):
     assert free0 - torch.cuda.mem_get_info()[0] < 1 << 20
     p.close()
     q.close()
+
+
+def test_data_that_do_not_fit_leave_nothing_to_train_on(cuda):
+    """A data set too large for the device's memory is refused, and training
+    is refused after it (the rows of the one before are gone)."""
+    from libbi_b200 import LearnedProposal, ModelL96
+    from libbi_b200 import _native as N
+
+    p = LearnedProposal(ModelL96(dim=40), 0.05, 128, 5)
+    data = _data(200, 13)
+    p.set_data(*data)
+    ptrs = [t.data_ptr() for t in data]
+    assert N.lib().bpf_proposal_set_data(p.handle, *ptrs, 2**31 - 1) == N.BPF_E_NOMEM  # 344 GB of means
+    assert N.lib().bpf_proposal_train(p.handle, 1, 64, 1e-3, None) == N.BPF_E_INVALID
+    p.set_data(*data)
+    assert np.isfinite(p.train(2, 64, 1e-3)).all()
+    p.close()
