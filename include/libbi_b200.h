@@ -447,6 +447,11 @@ int bpf_batch_set_seeds(bpf_batch* b, const uint64_t* seeds);
  * 256, 512, 1024 with the kept cluster size, infinite for a count that could
  * not be launched; may be NULL) report the state. */
 int bpf_batch_resample_threads(bpf_batch* b, int threads, int* current, double* tuned_us);
+/* The CTAs of a filter's cluster in the batched resampler (1, 2, 4 or 8; no
+ * counterpart in the reference).  ctas != 0 pins a size that holds the largest
+ * filter (BPF_E_INVALID for any other; a captured filter run is recaptured);
+ * current (may be NULL) reports the size in use. */
+int bpf_batch_resample_cluster(bpf_batch* b, int ctas, int* current);
 /* One BootstrapPF::step of every filter (see bpf_step); y_device: device
  * observations, nfilters x (dim for L96, 1 for PZ), filter-major, in the
  * model precision, or NULL for an unobserved step.  Does not synchronise. */

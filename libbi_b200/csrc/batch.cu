@@ -709,6 +709,20 @@ int bpf_batch_resample_threads(bpf_batch* b, int threads, int* current, double* 
   return BPF_OK;
 }
 
+int bpf_batch_resample_cluster(bpf_batch* b, int ctas, int* current) {
+  if (!b) return BPF_E_INVALID;
+  if (ctas != 0) {
+    if (!bpf::batch_resample_holds(b->rs, ctas)) return BPF_E_INVALID;
+    if (ctas != b->rs.group && b->graph) {
+      cudaGraphExecDestroy(b->graph);  // the captured steps launch the other size
+      b->graph = nullptr;
+    }
+    b->rs.group = ctas;
+  }
+  if (current) *current = b->rs.group;
+  return BPF_OK;
+}
+
 int bpf_batch_set_seeds(bpf_batch* b, const uint64_t* seeds) {
   if (!b || !seeds) return BPF_E_INVALID;
   for (int f = 0; f < b->nf; ++f) b->filt[f].seed = seeds[f];

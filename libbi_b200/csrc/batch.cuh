@@ -40,6 +40,8 @@ struct ResamplePlan {
   int group = 1;      // CTAs per filter (one thread-block cluster)
   int threads = 1024; // per CTA
 };
+// whether clusters of `group` CTAs hold the plan's largest filter
+bool batch_resample_holds(const ResamplePlan& p, int group);
 // fills all of the plan but order and sorted
 void plan_batch_resample(const BatchFilter* filt, int nf, ResamplePlan* p);
 int launch_batch_resample(const double* lw, int* as, const ResamplePlan& p, StepStats* stats, double* lu_buf,

@@ -481,13 +481,16 @@ static int launch_nt(const double* lw, int* as, const ResamplePlan& p, StepStats
   return BPF_OK;
 }
 
+bool batch_resample_holds(const ResamplePlan& p, int group) {
+  return p.max_n > 0 && p.max_n <= BPF_BATCH_MAX_PARTICLES && group >= 1 && group <= kGroup &&
+         (group & (group - 1)) == 0 && chunk_of(p.max_n, group) <= kCtaParticles;
+}
+
 // threads per CTA: 256, 512 or 1024 (the in-CTA arithmetic is exact, so the
 // count changes the speed only)
 int launch_batch_resample(const double* lw, int* as, const ResamplePlan& p, StepStats* stats,
                           double* lu_buf, int* os_buf, int step, cudaStream_t st) {
-  if (p.nf <= 0 || p.max_n <= 0 || p.max_n > BPF_BATCH_MAX_PARTICLES || p.group < 1 || p.group > kGroup ||
-      chunk_of(p.max_n, p.group) > kCtaParticles)
-    return BPF_E_INVALID;
+  if (p.nf <= 0 || !batch_resample_holds(p, p.group)) return BPF_E_INVALID;
   switch (p.threads) {
     case 256: return launch_nt<256>(lw, as, p, stats, lu_buf, os_buf, step, st);
     case 512: return launch_nt<512>(lw, as, p, stats, lu_buf, os_buf, step, st);

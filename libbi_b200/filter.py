@@ -567,6 +567,15 @@ class BatchedBootstrapPF:
                                                    us.ctypes.data_as(ctypes.c_void_p)), "bpf_batch_resample_threads")
         return cur.value, {256: us[0], 512: us[1], 1024: us[2]}
 
+    def resample_cluster(self, ctas: int = 0):
+        """CTAs of a filter's cluster in the resampler: pin 1, 2, 4 or 8 (of
+        those that hold the largest filter, 4096 particles a CTA), or 0 to
+        keep the autotuned size; returns the size in use."""
+        cur = ctypes.c_int()
+        N.check(N.lib().bpf_batch_resample_cluster(self._h, int(ctas), ctypes.byref(cur)),
+                "bpf_batch_resample_cluster")
+        return cur.value
+
     def set_proposal(self, proposal):
         """Attach a LearnedProposal to every filter (or None to detach):
         observed steps then run the guided step for the whole batch."""

@@ -2,6 +2,8 @@
 log-weights that stress them, against the oracle: ancestors equal as whole
 numbers (each is a function of exact sums of the same fixed-point weights, or
 of the same comparisons, so nothing is left to a tolerance)."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -47,10 +49,12 @@ def _own_uniforms(oracle, kind, n, seed, step):
 @pytest.mark.parametrize("max_n", [4096, 8192, 16384, 32768])
 def test_batch_resampler_at_cluster_and_run_edges(cuda, oracle, max_n):
     """Every kind at sizes around the runs of 16, the thread counts and the
-    CTAs' shares, in batches whose largest filter needs clusters of 1, 2, 4
-    and 8 CTAs (small filters then leave CTAs of their cluster empty)."""
+    CTAs' shares, with every cluster size that holds the largest filter (1 to
+    8 CTAs; small filters leave CTAs of their cluster empty) and every thread
+    count."""
     import torch
     from libbi_b200 import BatchedBootstrapPF, ModelPZ
+    from libbi_b200 import _native as N
 
     sizes = [2, 15, 17, 128, 129, 513, 1024, 4095, max_n - 1, max_n]
     ns = [n for n in sizes for _ in KINDS]
@@ -58,7 +62,13 @@ def test_batch_resampler_at_cluster_and_run_edges(cuda, oracle, max_n):
     seeds = [70 + f for f in range(len(ns))]
     batch = BatchedBootstrapPF([ModelPZ()] * len(ns), ns, kinds, seeds, ess_rel=1.0, metropolis_steps=B)
     y = torch.full((len(ns), 1), 0.5, dtype=torch.float64, device="cuda")
-    for threads, pattern in ((256, "spread"), (512, "one"), (1024, "few"), (256, "few"), (1024, "one")):
+    clusters = [g for g in (1, 2, 4, 8) if max_n <= 4096 * g]
+    for ctas in {1, 2, 3, 4, 16} - set(clusters):
+        with pytest.raises(N.BpfError):
+            batch.resample_cluster(ctas)
+    for i, (ctas, threads) in enumerate(itertools.product(clusters, (256, 512, 1024))):
+        pattern = ("spread", "one", "few")[(i + i // 3) % 3]
+        assert batch.resample_cluster(ctas) == ctas
         batch.resample_threads(threads)
         batch.init()
         batch.step_device(0.0, 1.0, y)
@@ -76,7 +86,7 @@ def test_batch_resampler_at_cluster_and_run_edges(cuda, oracle, max_n):
         got = anc.cpu().numpy()
         for f, n in enumerate(ns):
             want = _want(oracle, kinds[f], given[f], _own_uniforms(oracle, kinds[f], n, seeds[f], 2))[1]
-            np.testing.assert_array_equal(got[offs[f]:offs[f] + n], want, err_msg=f"{kinds[f]} {n} {pattern} {threads}")
+            np.testing.assert_array_equal(got[offs[f]:offs[f] + n], want, err_msg=f"{kinds[f]} {n} {pattern} {ctas} {threads}")
     batch.close()
 
 
