@@ -190,28 +190,33 @@ __device__ __forceinline__ int upper_bound_in(const T* __restrict__ A, int lo, i
 }
 
 // K searches per thread side by side, so that their loads are in flight
-// together: answers in [b, b + len], the same len for all.
+// together: answers in [first, first + len], the same range for all.
 template <int K, class T>
-__device__ __forceinline__ void block_upper_bounds(const T* __restrict__ A, int n, const T (&x)[K], T x_first, T x_last,
-                                                   int (&b)[K]) {
-  int bound[2];
-  block_bounds(A, n, x_first, x_last, bound);
-  int len = bound[1] - bound[0];
+__device__ __forceinline__ void upper_bounds_between(const T* __restrict__ A, int first, int len, const T (&x)[K],
+                                                     int (&b)[K]) {
 #pragma unroll
-  for (int k = 0; k < K; ++k) b[k] = bound[0];
+  for (int k = 0; k < K; ++k) b[k] = first;
   while (len > 1) {
     const int half = len >> 1;
     T v[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = __ldg(A + b[k] + half - 1);
+    for (int k = 0; k < K; ++k) v[k] = A[b[k] + half - 1];
 #pragma unroll
     for (int k = 0; k < K; ++k) b[k] = v[k] > x[k] ? b[k] : b[k] + half;
     len -= half;
   }
   if (len == 1) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) b[k] += __ldg(A + b[k]) > x[k] ? 0 : 1;
+    for (int k = 0; k < K; ++k) b[k] += A[b[k]] > x[k] ? 0 : 1;
   }
+}
+
+template <int K, class T>
+__device__ __forceinline__ void block_upper_bounds(const T* __restrict__ A, int n, const T (&x)[K], T x_first, T x_last,
+                                                   int (&b)[K]) {
+  int bound[2];
+  block_bounds(A, n, x_first, x_last, bound);
+  upper_bounds_between(A, bound[0], bound[1] - bound[0], x, b);
 }
 
 __device__ __forceinline__ bool gate_closed(const int* gate, const StepStats* st) {
@@ -1243,21 +1248,38 @@ k_permute_survivors(const int* __restrict__ Os, int n, const int* zprefix, int* 
 
 // Childless slot of rank r receives the ancestor a with E_a <= r < E_{a+1}.
 // One thread per rank, so the work is balanced however the copies are
-// distributed.
+// distributed.  Bound by the latency of the search's dependent loads: the
+// part of E that brackets a block's ranks is fetched into shared memory when
+// it fits (256 or 1024 ranks lie among some 700 or 2600 particles).
+constexpr int kStage = 4096;
 template <int K>
 __global__ void __launch_bounds__(kBlock)
 k_permute_fill(int* as, const int* __restrict__ E, const int* __restrict__ slot, const int* zprefix, int n, int T,
                const StepStats* st, const int* gate) {
   if (gate_closed(gate, st)) return;
+  __shared__ int s_E[kStage];
   const int R = zprefix[T];
   constexpr int kSpan = kBlock * K;
   for (long long b0 = (long long)blockIdx.x * kSpan; b0 < R; b0 += (long long)gridDim.x * kSpan) {
-    int r[K], b[K];
+    int r[K], b[K], to[K], bound[2];
 #pragma unroll
-    for (int k = 0; k < K; ++k) r[k] = (int)min(b0 + k * kBlock + threadIdx.x, (long long)R - 1);
-    block_upper_bounds(E, n, r, (int)b0, (int)min(b0 + kSpan, (long long)R) - 1, b);
+    for (int k = 0; k < K; ++k) {
+      r[k] = (int)min(b0 + k * kBlock + threadIdx.x, (long long)R - 1);
+      to[k] = __ldg(slot + r[k]);
+    }
+    block_bounds(E, n, (int)b0, (int)min(b0 + kSpan, (long long)R) - 1, bound);
+    const int len = bound[1] - bound[0];
+    if (len <= kStage) {
+      for (int i = threadIdx.x; i < len; i += kBlock) s_E[i] = __ldg(E + bound[0] + i);
+      __syncthreads();
+      upper_bounds_between(s_E, 0, len, r, b);
 #pragma unroll
-    for (int k = 0; k < K; ++k) as[__ldg(slot + r[k])] = b[k] - 1;
+      for (int k = 0; k < K; ++k) b[k] += bound[0];
+    } else {
+      upper_bounds_between(E, bound[0], len, r, b);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) as[to[k]] = b[k] - 1;
   }
 }
 

@@ -170,3 +170,26 @@ def test_stand_alone_resamplers_at_their_wide_forms(cuda, oracle, n):
                 np.testing.assert_array_equal(got, want[permute], err_msg=f"{kind} {pattern} permute={permute}")
     for r, _ in made.values():
         r.close()
+
+
+@pytest.mark.parametrize("n,s", [(100003, 16), (100003, 17), (400003, 4), (400003, 5)])
+def test_childless_slots_spread_thinly(cuda, oracle, n, s):
+    """Every s-th particle takes its neighbour as ancestor, so a block's 256
+    ranks (1024 with four searches per thread) are bracketed by 255 s (1023 s)
+    particles: just within and just beyond the 4096 that the fill of the
+    childless slots keeps in shared memory."""
+    import torch
+    from libbi_b200 import MetropolisResampler
+
+    lw = np.zeros(n)
+    target = np.arange(n)
+    target[: n - 1: s] += 1
+    u = np.empty(2 * n)
+    u[0::2] = (target + 0.5) / n  # the proposed ancestor
+    u[1::2] = 0.5  # accepted: log u < 0
+    r = MetropolisResampler(max_n=n, B=1)
+    plain = oracle.metropolis(lw, 1, u, 0)[1]
+    np.testing.assert_array_equal(plain, target)
+    got = r.ancestors(torch.as_tensor(lw, device="cuda"), torch.as_tensor(u, device="cuda"), permute=True)
+    np.testing.assert_array_equal(got.cpu().numpy(), oracle.permute_rule(plain))
+    r.close()
