@@ -8,8 +8,9 @@
 //                   the accumulators in tensor memory; only the tile's share
 //                   of the weight gradients (147 KB), its bias sums and its
 //                   loss leave the SM;
-//   k_reduce_adam   adds the shares in tile order, applies Adam and refreshes
-//                   the BF16 copy and the shared-memory images of the weights.
+//   k_reduce_adam   adds the shares in the order of the CTAs, applies Adam and
+//                   refreshes the BF16 copy and the shared-memory images of
+//                   the weights.
 // Layer by layer (eight dense launches with transposed staging, three split-K
 // reductions and nine small kernels, every activation through memory) a step
 // of 8192 rows took 510 us, most of it in kernels of 64 CTAs that staged
@@ -26,9 +27,11 @@
 // back-propagated errors, which contract over a weight image's rows, need no
 // transposed copies.
 //
-// The sums keep the order of the layer-by-layer form (128 rows per tile in
-// K steps of 16, tiles in order; biases in chunks of 64 rows in order), so
-// training is reproducible bit for bit.
+// Every sum has a fixed order, so training is reproducible bit for bit: a
+// weight gradient 128 rows at a time in K steps of 16, up to 148 tiles in the
+// order of the tiles (that of the layer-by-layer form); beyond, CTA c adds
+// tiles c, c + 148, ... in tensor memory, and the CTAs' shares are added in
+// order.  Bias gradients in chunks of 64 rows, in order.
 #include "internal.cuh"
 #include "tc.cuh"
 #include "proposal.cuh"
@@ -433,8 +436,8 @@ __global__ void __launch_bounds__(64) k_reduce_adam(ReduceAdamArgs a) {
   for (; k < terms; ++k) g += src[k * stride];
   a.grads[i] = g;
   if (!a.P) return;
-  // rounded as k_adam's expressions are compiled (proposal.cu), so that a run
-  // is the same whichever of the two steps it takes
+  // the fused products are spelled out: the moments' bits are then the same
+  // whatever the compiler makes of the sums
   const float m = __fmaf_rn(1.0f - a.b1, g, __fmul_rn(a.b1, a.M1[i]));
   const float v = __fmaf_rn(__fmul_rn(1.0f - a.b2, g), g, __fmul_rn(a.b2, a.M2[i]));
   a.M1[i] = m;
