@@ -10,7 +10,8 @@ particles for one observation interval.  Metric: particle-steps/s.
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
 Under torchrun each rank runs an independent replica (the single filter does
-not shard; replicas only) and rank 0 prints one JSON line.
+not shard; replicas only) and rank 0 prints one JSON line; the sections beside
+the headline go to standard error.
 """
 from __future__ import annotations
 
@@ -55,6 +56,21 @@ TRANSITION_FLOP_PER_PARTICLE = 5 * DIM * 31 + 2 * DIM + 6 * DIM
 # 128-thread blocks): 10.8 MB read, nothing written back within the launch
 # (the new state stays in L2)
 TRANSITION_DRAM_BYTES_PER_LAUNCH = 10_814_464 + 0
+
+
+# the sections beside the headline: tens of kilobytes, so they go to standard
+# error as one JSON object {"detail": ...}, and the line on standard output
+# stays short enough for a reader that keeps its last few kilobytes
+DETAIL = ("autotune", "kernels_large_n", "step_forms", "pz_c1", "batched", "pmmh", "precision", "precision_batched",
+          "guided")
+
+
+def split_detail(line):
+    """Take the sections of DETAIL out of the line; returns them."""
+    detail = {k: line.pop(k) for k in DETAIL if k in line}
+    if detail:
+        line["detail"] = sorted(detail)
+    return detail
 
 
 def peaks():
@@ -1428,6 +1444,9 @@ def main():
         dist.barrier()
         dist.destroy_process_group()
     if rank == 0:
+        detail = split_detail(line)
+        if detail:
+            print(json.dumps({"detail": detail}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     return 0
 

@@ -37,3 +37,19 @@ def test_reference_arm_other_ranks_print_nothing():
     r = _run({"RANK": "1", "WORLD_SIZE": "2", "LOCAL_RANK": "1"})
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.strip() == ""
+
+
+def test_own_arm_line_is_short():
+    """The line on standard output holds the contract's keys and names the
+    sections that went to standard error."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    line = {"metric": bench.METRIC, "value": 1.0, "e2e": {"value": 1.0}, "clocks": {}, "cpu_baseline": {"value": 1.0}}
+    sections = {k: {"x": "y" * 20000} for k in bench.DETAIL}
+    line.update(sections)
+    assert bench.split_detail(line) == sections
+    assert line["detail"] == sorted(bench.DETAIL)
+    assert set(line) == {"metric", "value", "e2e", "clocks", "cpu_baseline", "detail"}
+    headline = {"metric": bench.METRIC, "value": 1.0}
+    assert bench.split_detail(headline) == {} and "detail" not in headline
