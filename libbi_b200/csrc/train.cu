@@ -29,9 +29,9 @@
 //
 // Every sum has a fixed order, so training is reproducible bit for bit: a
 // weight gradient 128 rows at a time in K steps of 16, up to 148 tiles in the
-// order of the tiles (that of the layer-by-layer form); beyond, CTA c adds
-// tiles c, c + 148, ... in tensor memory, and the CTAs' shares are added in
-// order.  Bias gradients in chunks of 64 rows, in order.
+// order of the tiles; beyond, CTA c adds tiles c, c + 148, ... in tensor
+// memory, and the CTAs' shares are added in order.  Bias gradients in chunks
+// of 64 rows, in order.
 #include "internal.cuh"
 #include "tc.cuh"
 #include "proposal.cuh"

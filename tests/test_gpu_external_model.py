@@ -50,8 +50,8 @@ def _compare(pf, want, n):
 def test_test_bi_model_matches_oracle(cuda, oracle, model_libs, precision, n, resampler, B):
     """The reference's Test.bi (AR(1)) with an observation block, in the
     generated form, through bpf_create_model: every increment, the ESS and
-    the final state against the oracle, with the one-CTA (n <= 4096) and
-    grid-wide resamplers."""
+    the final state against the oracle, with the cluster (up to 4096
+    particles) and grid-wide resamplers."""
     from libbi_b200 import BootstrapPF
 
     model = _ar1(model_libs, precision)
