@@ -26,13 +26,15 @@ class HostSlots {
   // a slot of the caller's own, or null
   T* acquire() {
     std::lock_guard<std::mutex> lk(mu_);
-    if (block_ && used_ == 0 && !valid_(block_)) block_ = nullptr;
+    if (block_ && !valid_(block_)) {  // the slots in use went with it
+      block_ = nullptr;
+      for (bool& t : taken_) t = false;
+    }
     if (!block_) block_ = static_cast<T*>(alloc_(N * sizeof(T)));
     if (!block_) return nullptr;
     for (int i = 0; i < N; ++i)
       if (!taken_[i]) {
         taken_[i] = true;
-        ++used_;
         return block_ + i;
       }
     return nullptr;
@@ -42,10 +44,8 @@ class HostSlots {
   void release(T* slot) {
     if (!slot) return;
     std::lock_guard<std::mutex> lk(mu_);
-    const ptrdiff_t i = slot - block_;
-    if (i < 0 || i >= N || !taken_[i]) return;
-    taken_[i] = false;
-    --used_;
+    for (int i = 0; block_ && i < N; ++i)
+      if (slot == block_ + i) taken_[i] = false;
   }
 
  private:
@@ -54,7 +54,6 @@ class HostSlots {
   std::mutex mu_;
   T* block_ = nullptr;
   bool taken_[N] = {};
-  int used_ = 0;
 };
 
 }  // namespace bpf

@@ -36,9 +36,16 @@ int main() {
       s.release(p);
     }
     CHECK(allocs == 1);
-    // a block that went while nothing used it is replaced
+    // a block that went is replaced, also while a slot of it is held
     gone = true;
-    CHECK(s.acquire() && allocs == 2);
+    long long* p = s.acquire();
+    CHECK(p && allocs == 2);
+    gone = true;
+    long long* q = s.acquire();
+    CHECK(q && q != p && allocs == 3);
+    s.release(p);
+    for (int i = 0; i < 7; ++i) CHECK(s.acquire());
+    CHECK(!s.acquire());
   }
   {  // distinct slots, none left after the last, one again after a release
     Slots s(fake_alloc, fake_valid);
@@ -49,7 +56,7 @@ int main() {
     s.release(nullptr);
     s.release(*held.begin());
     CHECK(s.acquire() == *held.begin());
-    CHECK(allocs == 3);
+    CHECK(allocs == 4);
   }
   {  // no pinned memory: no slot, and a later try may succeed
     Slots s(fake_alloc, fake_valid);
